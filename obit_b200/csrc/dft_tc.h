@@ -1,0 +1,96 @@
+// Tensor-core form of the DFT model (dft_tc.cu): plan types shared by the host
+// planner (dft_tc_plan.cpp, plain C++) and the kernel.
+#pragma once
+#include <string>
+#include <vector>
+
+#include "dft_plan.h"
+
+namespace obit {
+
+constexpr int kTcChunk = 32;     // components per folded chunk
+constexpr int kTcMaxTeam = 2;    // warps (segments) of one record sharing its (record, component) work
+constexpr int kTcMinComps = 48;  // below this the recurrence kernels run (chunks would be mostly padding)
+
+// One warp's share of a record: a grid of rows x columns of channels,
+// channel(a, n) = ch0 + D a + n, valid below end.  Frequencies
+// are ratios to the data's reference frequency divided by 2 pi, so that a
+// product with X u + Y v + Z w is in turns.
+struct TcSeg {
+  float fa_hi, fa_lo;  // anchor: row 8 (MA - 1) + 4, column 4
+  int ch0;             // channel-list index of row 0, column 0; column n is n channels on
+  int end;             // first channel-list index past the segment (<= ch0: an empty segment)
+  int expo;            // float offset of the segment's exponent tables (TcExpo), spectra and tapers
+  float lam0, xi0;        // log-frequency term and squared frequency ratio at the reference channel
+};
+
+// A team of up to kTcMaxTeam segments of one uniformly spaced run (same steps).
+struct TcTeamDesc {
+  float w_hi, w_lo;    // row step: D channel increments
+  float w8_hi, w8_lo;  // eight rows
+  float s_hi, s_lo;    // channel increment
+  int D;
+  TcSeg seg[kTcMaxTeam];
+};
+
+// Float offsets inside a segment's exponent tables: the log-frequency term is
+// L(a, n) = lam0 + lamRow(a) + lamCol(n) + R(a, n), the squared frequency ratio
+// xi0 + xiRow(a) + xiCol(n) + xf(a) y(n), and R(a, n) ~ xl(a) y(n).
+struct TcExpo {
+  int lamRow, xiRow, xl, xf, lamCol, xiCol, y, L, total;
+};
+inline TcExpo tc_expo_layout(int MA, int NJ) {
+  TcExpo e{};
+  int o = 0;
+  auto take = [&](int n) { const int at = o; o += (n + 3) & ~3; return at; };
+  e.lamRow = take(16 * MA);
+  e.xiRow = take(16 * MA);
+  e.xl = take(16 * MA);
+  e.xf = take(16 * MA);
+  e.lamCol = take(8 * NJ);
+  e.xiCol = take(8 * NJ);
+  e.y = take(8 * NJ);
+  e.L = take(128 * MA * NJ);  // L(a, n) - lam0, in the order the lanes hold their sums
+  e.total = o;
+  return e;
+}
+
+// Kernel parameters.  Record and application fields as in KParams.
+struct TcParams {
+  KParams k;                // vis, nvis, lrec, iloc*, incs, pol*, op, ..., comps, ncomp, cstride, compsLo
+  const TcTeamDesc* teams;
+  int nteam;
+  const int* chanOff;       // record float offset of each selected channel's first polarization
+  const float* expo;
+  TcExpo lay;
+  int specField;            // component field of the spectral index
+};
+
+struct TcPlan {
+  bool on = false;
+  int MA = 2, NJ = 2, T = 1;  // 16 MA rows x 8 NJ columns per warp, T warps per team
+  int kind = kPoint;        // family of the (remaining) table: Point, PointSpec, Gauss, GaussSpec
+  int mixed = 0;            // a point sub-table precedes the Gaussian rows (as ModelDesc.ncompPt)
+  bool crossPt = false;     // point rows with a spectral index need the cross product
+  std::vector<TcTeamDesc> teams;
+  std::vector<int> chanOff;
+  std::vector<float> expo;
+  // device copies (one allocation) and launch facts
+  void* d_mem = nullptr;
+  TcParams kp{};
+  int gridCap = 0;
+};
+
+// Host part: whether the tensor-core form takes this layout and model, and its
+// teams and tables.  table: host copy of the table the kernels read (ncompPt
+// point rows first when mixed), rows of comp_stride floats.  Leaves plan->on
+// false (and returns) when the recurrence kernels should run.
+void tc_plan_layout(const LayoutDesc& L, const ModelDesc& M, const Plan& recur, const float* table, TcPlan* plan);
+
+// Device side and launch.
+int tc_finalize(TcPlan* plan, const KParams& base, std::string* err);
+void tc_free(TcPlan* plan);
+int tc_launch(const TcPlan& plan, const Plan& recur, float* d_vis, int nvis, const float* d_comps, int* d_err,
+              cudaStream_t stream, std::string* err);
+
+}  // namespace obit

@@ -1,0 +1,237 @@
+// Host planning of the tensor-core form (dft_tc.cu): uniformly spaced runs of
+// the selected channels, the warps' grids of rows x columns, the exponent
+// tables and their bounds, and the choice between this form and the
+// recurrence kernels.  Plain C++, no CUDA calls.
+#include <algorithm>
+#include <cmath>
+
+#include "dft_tc.h"
+
+namespace obit {
+
+namespace {
+
+// Largest neglected relative amplitude of a term (the corner of a segment's
+// grid; a fifth of it or less in the mean square): the rank-one residual
+// (alpha - alpha_t) R without the cross product, and the second order of the
+// cross exponent with it.
+constexpr double kTcResidualTol = 2.5e-6;
+// Without the cross product the exponents (alpha - alpha_t) lam of rows and
+// columns are taken to first order: x^2 / 2 at most this.
+constexpr double kTcFirstTol = 1.5e-7;
+
+struct Run {
+  double f0, df;  // frequency ratios f0 + k df
+  int list0, n;   // channel-list range
+  double lnShift; // log-frequency term = ln f + lnShift
+};
+
+void split_ds(double x, float* hi, float* lo) {
+  *hi = (float)x;
+  *lo = (float)(x - (double)*hi);
+}
+
+// Cost of one team per 8 components in scheduler cycles of the chip, from the
+// measured rates of full teams of points (1024, 512, 256 and 128 channels: 11.3,
+// 10.8, 8.6 and 5.8 T evaluations/s), against kRecurCost per channel of
+// the recurrence kernels' blocks (4.6-4.8 T).  With a spectral index the shapes measured 7.5,
+// 7.3, 6.8 and 4.7 T, in the same order.
+struct Shape {
+  int MA, NJ, T;
+  double cost;
+};
+constexpr Shape kShapes[] = {{2, 2, 2, 792.0}, {2, 2, 1, 416.0}, {1, 2, 1, 261.0}, {1, 1, 1, 192.0}};
+constexpr double kRecurCost = 1.9;
+
+bool spec_kind(int kind) { return kind == kPointSpec || kind == kGaussSpec; }
+bool gauss_kind(int kind) { return kind == kGauss || kind == kGaussSpec; }
+
+// Half the largest spread of the spectral index within a chunk.
+double chunk_spread(const float* table, int stride, int field, int ncomp) {
+  double s = 0.0;
+  for (int c0 = 0; c0 < ncomp; c0 += kTcChunk) {
+    const int c1 = std::min(ncomp, c0 + kTcChunk) - 1;
+    const double at = 0.5 * ((double)table[(size_t)c0 * stride + field] + (double)table[(size_t)c1 * stride + field]);
+    for (int c = c0; c <= c1; c++) s = std::max(s, std::fabs((double)table[(size_t)c * stride + field] - at));
+  }
+  return s;
+}
+
+double max_abs(const float* table, int stride, int field, int ncomp) {
+  double s = 0.0;
+  for (int c = 0; c < ncomp; c++) s = std::max(s, std::fabs((double)table[(size_t)c * stride + field]));
+  return s;
+}
+
+}  // namespace
+
+void tc_plan_layout(const LayoutDesc& L, const ModelDesc& M, const Plan& recur, const float* table, TcPlan* plan) {
+  *plan = TcPlan();
+  const bool spec = spec_kind(M.kind), gauss = gauss_kind(M.kind);
+  if (!(M.kind == kPoint || M.kind == kGauss || (spec && M.nterm == 1))) return;
+  const int npt = M.ncompPt, ntot = npt + M.ncomp;
+  if (ntot < kTcMinComps || M.ncomp < 1 || !table) return;
+  const int stride = comp_stride(M);
+  const int used = gauss ? (spec ? 8 : 7) : (spec ? 5 : 4);
+  for (int c = 0; c < ntot; c++) {
+    const float* r = table + (size_t)c * stride;
+    const int nf = c < npt ? 5 : used;
+    for (int i = 0; i < nf; i++)
+      if (!std::isfinite(r[i])) return;
+    // a taper never grows: g1 u^2 + g2 v^2 + g3 u v <= 0 for every u, v
+    if (gauss && c >= npt && !(r[4] <= 0.f && r[5] <= 0.f && 4.0 * r[4] * r[5] >= (double)r[6] * r[6] * (1.0 - 1e-5)))
+      return;
+  }
+
+  // ---- uniformly spaced runs of the selected channels -------------------------
+  std::vector<Run> runs;
+  std::vector<double> f;
+  std::vector<int> off;
+  std::vector<double> ln;
+  for (int iIF = L.ifb; iIF <= L.ife; iIF++)
+    for (int ch = L.chanb; ch <= L.chane; ch++) {
+      const int i = ch * L.kincf + iIF * L.kincif;
+      f.push_back(L.fscale[i]);
+      off.push_back(L.nrparm + iIF * L.incif + ch * L.incf + L.stokb * L.incs);
+      ln.push_back(spec ? L.lnspec[i] : 0.0);
+      if (!(L.fscale[i] > 0.0)) return;
+    }
+  const int n = (int)f.size();
+  for (int i = 0; i < n;) {
+    int e = i + 1;
+    double df = 0.0;
+    if (e < n) {
+      df = f[e] - f[i];
+      // the increment's own rounding grows with the run; the run is checked
+      // against its mean increment below
+      while (e < n && std::fabs(f[e] - (f[i] + (e - i) * df)) <= (1e-13 + 4.5e-16 * (e - i)) * f[i]) e++;
+    }
+    Run r{f[i], df, i, e - i, spec ? ln[i] - std::log(f[i]) : 0.0};
+    if (r.n > 1) r.df = (f[e - 1] - f[i]) / (r.n - 1);
+    for (int k = 0; k < r.n; k++) {
+      if (std::fabs(f[i + k] - (r.f0 + k * r.df)) > 2e-13 * f[i]) return;
+      if (spec && std::fabs(ln[i + k] - (std::log(f[i + k]) + r.lnShift)) > 1e-9) return;
+    }
+    runs.push_back(r);
+    i = e;
+  }
+
+  // ---- the cheapest shape that holds the bounds ---------------------------------
+  const double spreadPt = (gauss && npt) || (!gauss && spec)
+                              ? chunk_spread(table, stride, kSpecIndexField, gauss ? npt : M.ncomp) : 0.0;
+  const float* gt = table + (size_t)npt * stride;
+  const double spreadG = (gauss && spec) ? chunk_spread(gt, stride, 7, M.ncomp) : 0.0;
+  double amax = 0.0;
+  if (!gauss && spec) amax = max_abs(table, stride, kSpecIndexField, M.ncomp);
+  if (gauss && npt) amax = max_abs(table, stride, kSpecIndexField, npt);
+  if (gauss && spec) amax = std::max(amax, max_abs(gt, stride, 7, M.ncomp));
+  double best = kRecurCost * recur.kp.nblocks * recur.tune.K;  // its blocks are padded too
+  TcPlan chosen;
+  for (const Shape& s : kShapes) {
+    double cost = 0.0;
+    const int segCap = 128 * s.MA * s.NJ, cap = segCap * s.T;
+    for (const Run& r : runs) cost += s.cost * ((r.n + cap - 1) / cap);
+    if (!(cost < best)) continue;
+    TcPlan p;
+    p.MA = s.MA;
+    p.NJ = s.NJ;
+    p.T = s.T;
+    p.kind = M.kind;
+    p.mixed = npt > 0;
+    p.chanOff = off;
+    const TcExpo lay = tc_expo_layout(s.MA, s.NJ);
+    const int D = 8 * s.NJ, a0 = 8 * (s.MA - 1) + 4, rows = 16 * s.MA, cols = 8 * s.NJ;
+    const double inv2pi = 0.15915494309189533577;
+    bool ok = true;
+    double resid1 = 0.0, resid2 = 0.0, gcross = 0.0, range = 0.0;
+    for (const Run& r : runs) {
+      for (int t0 = 0; t0 < r.n && ok; t0 += cap) {
+        TcTeamDesc tm{};
+        tm.D = D;
+        split_ds(D * r.df * inv2pi, &tm.w_hi, &tm.w_lo);
+        split_ds(8.0 * D * r.df * inv2pi, &tm.w8_hi, &tm.w8_lo);
+        split_ds(r.df * inv2pi, &tm.s_hi, &tm.s_lo);
+        for (int q = 0; q < s.T; q++) {
+          TcSeg& g = tm.seg[q];
+          const int k0 = t0 + q * segCap;
+          auto F = [&](double x) { return r.f0 + (k0 + x) * r.df; };  // ratio at channel offset x of the segment
+          g.end = r.list0 + std::min(r.n, k0 + segCap);
+          split_ds(F(D * a0 + 4) * inv2pi, &g.fa_hi, &g.fa_lo);
+          g.ch0 = r.list0 + k0;
+          if (!(spec || gauss) || k0 >= r.n) continue;
+          if (!(std::min(F(0), F(segCap - 1)) > 0.05 * r.f0)) {
+            ok = false;
+            break;
+          }
+          // exponent tables: rows a against the middle column, columns n against the middle row
+          g.expo = (int)p.expo.size();
+          p.expo.resize(p.expo.size() + lay.total, 0.0f);
+          float* ex = p.expo.data() + g.expo;
+          const double nm = 0.5 * (cols - 1);
+          auto Lg = [&](double a, double nn) { return std::log(F(D * a + nn)) + r.lnShift; };
+          auto F2 = [&](double a, double nn) { const double x = F(D * a + nn); return x * x; };
+          const int last = std::min(r.n - k0, segCap) - 1;          // last valid channel offset
+          const double ar = r.df >= 0.0 ? 0.0 : (double)(last / D);  // row of the least taper
+          const double am = 0.5 * std::min<double>(rows - 1, (double)(last / D));  // middle valid row
+          const double lam0 = Lg(am, nm), xi0 = F2(ar, nm);
+          g.lam0 = (float)lam0;
+          g.xi0 = (float)xi0;
+          double yy = 0.0;
+          for (int c = 0; c < cols; c++) {
+            const double y = (c - nm) * r.df;
+            ex[lay.y + c] = (float)y;
+            ex[lay.lamCol + c] = spec ? (float)(Lg(am, c) - lam0) : 0.f;
+            ex[lay.xiCol + c] = (float)(F2(am, c) - F2(am, nm));
+            yy += y * y;
+          }
+          for (int a = 0; a < rows; a++) {
+            ex[lay.lamRow + a] = spec ? (float)(Lg(a, nm) - lam0) : 0.f;
+            ex[lay.xiRow + a] = (float)(F2(a, nm) - xi0);
+            ex[lay.xf + a] = (float)(2.0 * D * (a - am) * r.df);
+            double ry = 0.0, R[64];
+            for (int c = 0; c < cols && spec; c++) {
+              R[c] = Lg(a, c) - Lg(a, nm) - Lg(am, c) + lam0;
+              ry += R[c] * (c - nm) * r.df;
+              // fragment order: lane (row % 8) * 4 + (column % 8) / 2
+              const int mi = a >> 4, e = 2 * ((a >> 3) & 1) + (c & 1);
+              const int lane = 4 * (a & 7) + ((c & 7) >> 1);
+              ex[lay.L + ((mi * s.NJ + (c >> 3)) * 32 + lane) * 4 + e] = (float)(Lg(a, c) - lam0);
+            }
+            const double xl = (spec && yy > 0.0) ? ry / yy : 0.0;
+            ex[lay.xl + a] = (float)xl;
+            for (int c = 0; c < cols; c++) {
+              if (D * a + c > last) continue;
+              const double y = (c - nm) * r.df;
+              if (spec) {
+                resid1 = std::max(resid1, std::fabs(R[c]));
+                resid2 = std::max(resid2, std::fabs(R[c] - xl * y));
+                range = std::max(range, std::fabs(Lg(a, c) - lam0));
+              }
+              gcross = std::max(gcross, std::fabs(2.0 * D * (a - am) * r.df * y) / F2(a, c));
+            }
+          }
+        }
+        p.teams.push_back(tm);
+      }
+      if (!ok) break;
+    }
+    if (!ok) continue;
+    auto second = [&](double x) { return 0.5 * x * x; };
+    if (spec && amax * range > 8.0) continue;
+    if ((!gauss && spec) || npt) {
+      p.crossPt = spreadPt * resid1 > kTcResidualTol || second(spreadPt * range) > kTcFirstTol;
+      if (p.crossPt && std::max(spreadPt * resid2, second(spreadPt * resid1)) > kTcResidualTol) continue;
+    }
+    if (gauss) {
+      // second order of the taper's cross exponent q c times the taper exp(-q): largest at q = 2
+      if (0.2707 * gcross * gcross > kTcResidualTol) continue;
+      if (spec && std::max(spreadG * resid2, second(spreadG * resid1)) > kTcResidualTol) continue;
+    }
+    p.on = true;
+    best = cost;
+    chosen = std::move(p);
+  }
+  *plan = std::move(chosen);
+}
+
+}  // namespace obit

@@ -20,6 +20,7 @@
 #include "abi_internal.h"
 #include "dft_beam.h"
 #include "dft_plan.h"
+#include "dft_tc.h"
 
 namespace {
 
@@ -127,6 +128,7 @@ struct State {
   const float* runComps = nullptr;  // table the plan's launches read
   // plan
   Plan plan;
+  TcPlan tc;  // the tensor-core form, where it takes the plan's layout and model
   bool planValid = false;
   // staging
   int bufRows = 0;                 // rows per device staging buffer
@@ -171,6 +173,7 @@ int ensure_state(GPUInfo* g, State** out) {
 void release_state(State* s) {
   cudaSetDevice(s->device);
   free_plan(&s->plan);
+  tc_free(&s->tc);
   if (s->d_comps) cudaFree(s->d_comps);
   if (s->d_lo) cudaFree(s->d_lo);
   if (s->d_sorted) cudaFree(s->d_sorted);
@@ -192,10 +195,11 @@ void release_state(State* s) {
 //    matching point family's field order and ordered by index, followed by
 //    the Gaussian components.  *md becomes that point family when no Gaussian
 //    is left, else a mixed model (md->ncompPt point rows, md->ncomp Gaussian).
-// *index receives the ordered spectral indices of the point rows; left empty
-// (no copy made, *md unchanged) when an index is not finite or no component
-// qualifies.
-int prepare_run_table(State* s, ModelDesc* md, std::vector<float>* index) {
+// The Gaussian rows are ordered by index too.  *index receives the ordered
+// spectral indices of the point rows, *table the copy's rows on the host; both
+// left empty (no copy made, *md unchanged) when an index is not finite or no
+// component qualifies.
+int prepare_run_table(State* s, ModelDesc* md, std::vector<float>* index, std::vector<float>* table) {
   index->clear();
   const bool gauss = md->kind == kGaussSpec || md->kind == kGaussTSpec;
   const size_t stride = (size_t)comp_stride(*md), n = (size_t)md->ncomp;
@@ -216,9 +220,11 @@ int prepare_run_table(State* s, ModelDesc* md, std::vector<float>* index) {
     else gs.push_back((int)i);
   }
   if (pts.empty()) return OBIT_DFT_OK;
-  std::stable_sort(pts.begin(), pts.end(), [&](int a, int b) {
+  auto by_index = [&](int a, int b) {
     return tab[(size_t)a * stride + aField] < tab[(size_t)b * stride + aField];
-  });
+  };
+  std::stable_sort(pts.begin(), pts.end(), by_index);
+  std::stable_sort(gs.begin(), gs.end(), by_index);
   std::vector<float> out(tab.size(), 0.0f), outLo(lo.size());
   index->resize(pts.size());
   for (size_t k = 0; k < pts.size(); k++) {
@@ -266,6 +272,7 @@ int prepare_run_table(State* s, ModelDesc* md, std::vector<float>* index) {
       md->ncomp = (int)gs.size();
     }
   }
+  *table = std::move(out);
   return OBIT_DFT_OK;
 }
 
@@ -279,20 +286,21 @@ int ensure_plan(GPUInfo* g, State* s) {
   if (!rc) rc = apply_from_info(s->mc, s->pr, L, &A, &err);
   if (rc) return fail(rc, err);
   free_plan(&s->plan);
+  tc_free(&s->tc);
   // Point families with one spectral index: the recurrence kernels read a copy
   // ordered by the index, which lets the planner choose the spectral-factored
   // form (the wait-limit diagnostic has a chain-form instance only).
   TuneDesc T = s->tune;
   if (s->waitPolls != kDefaultWaitPolls) T.specFactor = 0;
   ModelDesc md = s->mc.model;
-  std::vector<float> index;
+  std::vector<float> index, table;
   s->runComps = s->d_comps;
   const float* runLo = s->haveLo ? s->d_lo : nullptr;
   const bool ptOne = md.kind == kPointTSpec || (md.kind == kPointSpec && md.nterm == 1);
   const bool gsOne = md.kind == kGaussTSpec || (md.kind == kGaussSpec && md.nterm == 1);
   if (T.flavor == kFlavorRecur && T.specFactor && md.ncomp > 1 && (ptOne || (gsOne && !s->haveLo))) {
     ModelDesc m2 = md;
-    if ((rc = prepare_run_table(s, &m2, &index))) return rc;
+    if ((rc = prepare_run_table(s, &m2, &index, &table))) return rc;
     if (!index.empty()) {
       m2.specIndex = index.data();
       Plan trial;
@@ -311,6 +319,16 @@ int ensure_plan(GPUInfo* g, State* s) {
   s->plan.kp.compsLo = runLo;
   if (!rc) rc = finalize_plan(&s->plan, nullptr, 0, &err);
   if (rc) return fail(rc, err);
+  // the tensor-core form, unless a kernel or tile shape was asked for
+  if (T.flavor == kFlavorRecur && T.specFactor && T.K == 0 && T.ct == 0 && T.Bt == 0 && T.threads == 0 &&
+      s->plan.linear && !s->beam.on && md.ncompPt + md.ncomp >= kTcMinComps) {
+    if (s->runComps == s->d_comps) {
+      table.resize((size_t)md.ncomp * comp_stride(md));
+      CUDA_TRY(cudaMemcpy(table.data(), s->d_comps, sizeof(float) * table.size(), cudaMemcpyDeviceToHost));
+    }
+    tc_plan_layout(L, md, s->plan, table.data(), &s->tc);
+    if (s->tc.on && (rc = tc_finalize(&s->tc, s->plan.kp, &err))) return fail(rc, err);
+  }
   if (s->beam.on) {  // launch parameters and per-(channel, IF) tables of the beam kernel
     BeamState& b = s->beam;
     if (b.jonesComps < s->mc.model.ncomp)
@@ -445,6 +463,12 @@ int ensure_plan(GPUInfo* g, State* s) {
   }
   s->planValid = true;
   return OBIT_DFT_OK;
+}
+
+// The plain sky model over nvis records at d_vis.
+int launch_model(State* s, float* d_vis, int nvis, cudaStream_t stream, std::string* err) {
+  if (s->tc.on) return tc_launch(s->tc, s->plan, d_vis, nvis, s->runComps, s->d_err, stream, err);
+  return launch_plan(s->plan, d_vis, 0, nvis, s->runComps, s->d_err, stream, err);
 }
 
 int read_err_flag(State* s) {
@@ -709,7 +733,7 @@ int obit_dft_calc_device(GPUInfo* g, float* d_vis, int nvis, void* stream) {
     k.k.nvis = nvis;
     rc = launch_beam(k, (cudaStream_t)stream, &err);
   } else {
-    rc = launch_plan(s->plan, d_vis, 0, nvis, s->runComps, s->d_err, (cudaStream_t)stream, &err);
+    rc = launch_model(s, d_vis, nvis, (cudaStream_t)stream, &err);
   }
   if (rc) return fail(rc, err);
   return OBIT_DFT_OK;
@@ -724,10 +748,10 @@ int obit_dft_plan_info(GPUInfo* g, int* info, int n) {
   rc = ensure_plan(g, s);
   if (rc) return rc;
   const Plan& pl = s->plan;
-  const int v[11] = {pl.tune.flavor, pl.tune.K, pl.kp.ct, pl.kp.Bt, pl.kp.R, pl.threads,
+  const int v[12] = {pl.tune.flavor, pl.tune.K, pl.kp.ct, pl.kp.Bt, pl.kp.R, pl.threads,
                      pl.kp.nblocks, pl.kp.ndf, pl.specFactored ? 1 : 0, pl.mixed ? 1 : 0,
-                     pl.mixed ? pl.model.ncompPt : 0};
-  for (int i = 0; i < n && i < 11; i++) info[i] = v[i];
+                     pl.mixed ? pl.model.ncompPt : 0, s->tc.on ? 128 * s->tc.MA * s->tc.NJ * s->tc.T : 0};
+  for (int i = 0; i < n && i < 12; i++) info[i] = v[i];
   return OBIT_DFT_OK;
 }
 
@@ -838,7 +862,7 @@ int obit_dft_calc(GPUInfo* g) {
       k.k.nvis = nr;
       rc = launch_beam(k, streams[b], &err, !beamPrologue);
     } else {
-      rc = launch_plan(s->plan, bufs[b], 0, nr, s->runComps, s->d_err, streams[b], &err);
+      rc = launch_model(s, bufs[b], nr, streams[b], &err);
     }
     if (rc) return fail(rc, err);
     CUDA_TRY(cudaMemcpyAsync(host, bufs[b], bytes, cudaMemcpyDeviceToHost, streams[b]));

@@ -193,10 +193,10 @@ class GPUSkyModel:
 
     def plan_info(self) -> dict:
         """The kernel plan the next call uses (built on demand)."""
-        arr = (C.c_int * 11)()
-        _lib.check(self._lib.obit_dft_plan_info(self.gpuinfo, arr, 11))
+        arr = (C.c_int * 12)()
+        _lib.check(self._lib.obit_dft_plan_info(self.gpuinfo, arr, 12))
         keys = ("flavor", "K", "ct", "Bt", "R", "threads", "nblocks", "ndf", "specFactored", "mixed",
-                "ncompPoint")
+                "ncompPoint", "tensorChannels")
         return dict(zip(keys, list(arr)))
 
     def beam_info(self) -> dict:

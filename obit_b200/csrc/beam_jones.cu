@@ -3,9 +3,9 @@
 // (ObitCUDABeamModel.cu:1228-1299) with its pixel geometry (CUDAPositionXYpix,
 // CUDASkyGeom.h:91-286; linear grids and the eight projections) and Lagrange interpolator
 // (CUDABeamInterpPixel / SetConvKernal, CUDABeamInterp.h), written anew.
-// One thread per (component, antenna type); the position, its pixel, the
-// interpolation kernels and the primary-beam factor's offset are computed
-// once, then every plane's 8 images are interpolated with the same taps.
+// The position, its pixel, the interpolation weights and the primary-beam
+// factor's offset are computed once per component, then every plane's 8 images
+// are interpolated with the same taps.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -150,24 +150,23 @@ __device__ bool pixel_of(const JonesParams& p, double x, double y, float& px, fl
   return true;
 }
 
-// Lagrange weights of the iwid taps about pixel (1-relative) on an axis of n
-// pixels; start: first tap (0-relative).
-__device__ void lagrange_taps(float pix, int n, int hw, int& start, float* w) {
+// First (0-relative) of the taps about pixel pix (1-relative) on an axis of n pixels.
+__device__ int first_tap(float pix, int n, int hw) {
   const int iwid = 2 * hw + 1;
-  const int ipos = (int)(pix + 0.5f);
-  int cen = ipos - hw;
-  cen = max(1, min(cen, n - iwid + 1)) - 1;
-  start = cen;
-  const float xx = pix - (float)cen;  // 1 at the first tap
-  for (int j = 0; j < iwid; j++) {
-    float prod = 1.0f, den = 1.0f;
-    for (int i = 0; i < iwid; i++)
-      if (i != j) {
-        prod *= xx - (float)(i + 1);
-        den *= (float)(j - i);
-      }
-    w[j] = prod / den;
-  }
+  const int cen = (int)(pix + 0.5f) - hw;
+  return max(1, min(cen, n - iwid + 1)) - 1;
+}
+
+// Lagrange weight of tap j of iwid whose first is `start`.
+__device__ float lagrange_weight(float pix, int start, int iwid, int j) {
+  const float xx = pix - (float)start;  // 1 at the first tap
+  float prod = 1.0f, den = 1.0f;
+  for (int i = 0; i < iwid; i++)
+    if (i != j) {
+      prod *= xx - (float)(i + 1);
+      den *= (float)(j - i);
+    }
+  return prod / den;
 }
 
 // Inverse square root of the cos^2 primary-beam gain at offset ang (deg):
@@ -178,63 +177,131 @@ __device__ float inv_beam(float fact, float freq, float ang) {
   return (float)((1.0 - 4.0 * arg * arg) / cos(3.141592653589793 * arg));
 }
 
-__device__ __forceinline__ void set_unit(float* J) {
-  J[0] = 1.f; J[1] = 0.f; J[2] = 0.f; J[3] = 0.f;
-  J[4] = 0.f; J[5] = 0.f; J[6] = 1.f; J[7] = 0.f;
+// a blank interpolant in the exchange between lanes: a NaN no arithmetic produces
+constexpr int kBlankBits = 0x7fc0beef;
+
+// Units: one interpolation of (component, plane, image).  A CTA takes CB
+// components of one antenna type: a thread per component finds the pixel, a
+// thread per tap its weight on an axis, all threads the (offset, weight) table, then eight lanes share a unit, each every eighth tap, and at last a
+// thread per (component, plane) applies the gain and the limits.  The images
+// come from L2 (1.9 MB at 2 types x 8 planes x 61 x 61 pixels); a warp's load
+// touches 4 units of two rows each.  A thread per (component, type) over all
+// planes, images and taps kept 8,000 threads on 200 dependent loads a plane:
+// 160 us for 4,000 components x 2 types x 8 planes of 61 x 61 pixels, now 41.
+constexpr int kJonesThreads = 256;
+constexpr int kMaxCB = 32;
+
+__host__ __device__ inline int jones_comps_per_cta(int nplane) {
+  const int cb = 2 * kJonesThreads / (8 * nplane);
+  return cb < 1 ? 1 : (cb > kMaxCB ? kMaxCB : cb);
 }
 
-__global__ void beam_jones_kernel(const __grid_constant__ JonesParams p) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  const int t = blockIdx.y;
-  if (c >= p.ncomp || t >= p.numAntType) return;
-  float* Jc = p.jones + ((size_t)t * p.ncomp + c) * p.nplane * 8;
-  const double x = p.pos[2 * c], y = p.pos[2 * c + 1];
-  float px, py;
-  const bool onGrid = pixel_of(p, x, y, px, py) && px >= 1.0f && px <= (float)p.nx && py >= 1.0f &&
-                      py <= (float)p.ny;
-  if (!onGrid) {
-    for (int k = 0; k < p.nplane; k++) set_unit(Jc + 8 * k);
-    return;
+__global__ void __launch_bounds__(kJonesThreads) beam_jones_kernel(const __grid_constant__ JonesParams p) {
+  __shared__ float sW[kMaxCB][2][kMaxTaps];
+  __shared__ int sFirst[kMaxCB];  // offset of the first tap, or -1 off the grid
+  __shared__ float sAng[kMaxCB], sSum[kMaxCB], sPix[kMaxCB][2];
+  extern __shared__ __align__(8) float dynJ[];
+  const int CB = jones_comps_per_cta(p.nplane);
+  const int iwid = 2 * p.hwidth + 1, ntap = iwid * iwid;
+  float2* sTap = reinterpret_cast<float2*>(dynJ);           // [CB][ntap]: offset (as bits), weight
+  float* sV = dynJ + 2 * CB * ntap;                         // [CB][nplane][8]
+  const int c0 = blockIdx.x * CB, t = blockIdx.y;
+  const int nc = min(CB, p.ncomp - c0);
+  if ((int)threadIdx.x < nc) {
+    const int i = threadIdx.x, c = c0 + i;
+    const double x = p.pos[2 * c], y = p.pos[2 * c + 1];
+    float px, py;
+    const bool onGrid = pixel_of(p, x, y, px, py) && px >= 1.0f && px <= (float)p.nx && py >= 1.0f &&
+                        py <= (float)p.ny;
+    sFirst[i] = onGrid ? first_tap(py, p.ny, p.hwidth) * p.nx + first_tap(px, p.nx, p.hwidth) : -1;
+    sPix[i][0] = px;
+    sPix[i][1] = py;
+    sAng[i] = sqrtf((float)(x * x + y * y));
   }
-  const int iwid = 2 * p.hwidth + 1;
-  int xs, ys;
-  float wx[kMaxTaps], wy[kMaxTaps];
-  lagrange_taps(px, p.nx, p.hwidth, xs, wx);
-  lagrange_taps(py, p.ny, p.hwidth, ys, wy);
-  const float ang = sqrtf((float)(x * x + y * y));
-  const size_t img = (size_t)p.nplane * p.ny * p.nx;
-  const float* base = p.pixels + (size_t)t * 8 * img;
-  for (int k = 0; k < p.nplane; k++) {
-    float v[8];
+  __syncthreads();
+  for (int e = threadIdx.x; e < nc * 2 * iwid; e += kJonesThreads) {  // a thread per tap of an axis
+    const int i = e / (2 * iwid), r = e - i * 2 * iwid, ax = r >= iwid, j = ax ? r - iwid : r;
+    if (sFirst[i] >= 0) {
+      const float pix = sPix[i][ax];
+      sW[i][ax][j] = lagrange_weight(pix, first_tap(pix, ax ? p.ny : p.nx, p.hwidth), iwid, j);
+    }
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < nc && sFirst[threadIdx.x] >= 0) {
+    const int i = threadIdx.x;
+    float s = 0.f;
+    for (int j = 0; j < iwid; j++)
+      for (int k = 0; k < iwid; k++) s += sW[i][0][k] * sW[i][1][j];
+    sSum[i] = s;
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < nc * ntap; e += kJonesThreads) {
+    const int i = e / ntap, k = e - i * ntap, j = k / iwid, m = k - j * iwid;
+    if (sFirst[i] >= 0)
+      sTap[e] = make_float2(__int_as_float(sFirst[i] + j * p.nx + m), sW[i][0][m] * sW[i][1][j]);
+  }
+  __syncthreads();
+  const size_t plane = (size_t)p.ny * p.nx;
+  const float* base = p.pixels + (size_t)t * 8 * p.nplane * plane;
+  const int units = nc * p.nplane * 8, l = threadIdx.x & 7;
+  for (int u0 = 0; u0 < units; u0 += kJonesThreads / 8) {
+    const int u = u0 + (threadIdx.x >> 3);
+    const int q = u & 7, ck = u >> 3, i = ck / p.nplane, k = ck - i * p.nplane;
+    const bool have = u < units && sFirst[min(i, CB - 1)] >= 0;
+    float sum = 0.f, sumwt = 0.f;
     bool blank = false;
-    for (int q = 0; q < 8; q++) {
-      const float* d = base + q * img + (size_t)k * p.ny * p.nx;
-      float sum = 0.f, sumwt = 0.f;
-      for (int j = 0; j < iwid; j++) {
-        const float* row = d + (size_t)(ys + j) * p.nx + xs;
-        for (int i = 0; i < iwid; i++) {
-          const float val = row[i];
-          if (val != p.fblank) {
-            const float wt = wx[i] * wy[j];
-            sumwt += wt;
-            sum += val * wt;
+    if (have) {
+      const float* d = base + ((size_t)q * p.nplane + k) * plane;
+      const float2* tap = sTap + i * ntap;
+      for (int e0 = l; e0 < ntap; e0 += 32) {  // four loads in flight per lane
+        float val[4], w[4];
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+          const int e = e0 + 8 * m;
+          const float2 tw = e < ntap ? tap[e] : make_float2(tap[l].x, 0.f);
+          w[m] = tw.y;
+          val[m] = __ldg(d + __float_as_int(tw.x));
+        }
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+          if (e0 + 8 * m >= ntap) continue;
+          if (val[m] != p.fblank) {
+            sumwt += w[m];
+            sum += val[m] * w[m];
+          } else {
+            blank = true;
           }
         }
       }
-      if (sumwt > 0.90f) v[q] = sum / sumwt;
-      else blank = true;
     }
-    const float g = inv_beam(p.refSizeFact, p.planeFreq[k], ang);
-    float* J = Jc + 8 * k;
-    if (blank || !(g < 10.0f) || !(fabsf(g * v[0]) <= 1.3f) || !(fabsf(g * v[2]) <= 1.3f)) {
-      set_unit(J);
-      continue;
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    float wt = have ? sSum[i] : 1.f;
+    if (__any_sync(0xffffffffu, blank)) {
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) sumwt += __shfl_xor_sync(0xffffffffu, sumwt, o);
+      wt = sumwt;
+    }
+    if (have && l == 0) sV[u] = wt > 0.90f ? sum / wt : __int_as_float(kBlankBits);
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < nc * p.nplane; e += kJonesThreads) {
+    const int i = e / p.nplane, k = e - i * p.nplane;
+    float* J = p.jones + (((size_t)t * p.ncomp + c0 + i) * p.nplane + k) * 8;
+    bool unit = sFirst[i] < 0;
+    float v[8], g = 0.f;
+    if (!unit) {
+      g = inv_beam(p.refSizeFact, p.planeFreq[k], sAng[i]);
+      for (int q = 0; q < 8; q++) {
+        v[q] = sV[e * 8 + q];
+        unit = unit || __float_as_int(v[q]) == kBlankBits;
+      }
+      unit = unit || !(g < 10.0f) || !(fabsf(g * v[0]) <= 1.3f) || !(fabsf(g * v[2]) <= 1.3f);
     }
     // cudaMatxSet2C order: P1, X1, X2, P2 (XX, XY, YX, YY)
-    J[0] = g * v[0]; J[1] = g * v[1];
-    J[2] = g * v[4]; J[3] = g * v[5];
-    J[4] = g * v[6]; J[5] = g * v[7];
-    J[6] = g * v[2]; J[7] = g * v[3];
+    float4* J4 = reinterpret_cast<float4*>(J);
+    J4[0] = unit ? make_float4(1.f, 0.f, 0.f, 0.f) : make_float4(g * v[0], g * v[1], g * v[4], g * v[5]);
+    J4[1] = unit ? make_float4(0.f, 0.f, 1.f, 0.f) : make_float4(g * v[6], g * v[7], g * v[2], g * v[3]);
   }
 }
 
@@ -284,8 +351,10 @@ extern "C" int obit_dft_beam_jones(const ObitDFTBeamImages* im, const float* pos
   for (int k = 0; k < im->nplane; k++) p.planeFreq[k] = im->planeFreq[k];
   cudaError_t ce = cudaGetLastError();
   if (ce != cudaSuccess) return bad(OBIT_DFT_ECUDA, cudaGetErrorString(ce));
-  const dim3 grid((unsigned)((ncomp + 127) / 128), (unsigned)im->numAntType);
-  beam_jones_kernel<<<grid, 128, 0, (cudaStream_t)stream>>>(p);
+  const int cb = jones_comps_per_cta(p.nplane), iwid = 2 * p.hwidth + 1;
+  const dim3 grid((unsigned)((ncomp + cb - 1) / cb), (unsigned)im->numAntType);
+  const size_t smem = sizeof(float) * ((size_t)2 * cb * iwid * iwid + (size_t)cb * p.nplane * 8);
+  beam_jones_kernel<<<grid, kJonesThreads, smem, (cudaStream_t)stream>>>(p);
   ce = cudaGetLastError();
   if (ce != cudaSuccess) {
     set_last_error(std::string("beam Jones kernel launch: ") + cudaGetErrorString(ce));

@@ -4,6 +4,7 @@
 #include <string>
 #include <vector>
 
+#include "dft_beam.h"
 #include "dft_plan.h"
 
 namespace obit {
@@ -20,6 +21,7 @@ struct TcSeg {
   float fa_hi, fa_lo;  // anchor: row 8 (MA - 1) + 4, column 4
   int ch0;             // channel-list index of row 0, column 0; column n is n channels on
   int end;             // first channel-list index past the segment (<= ch0: an empty segment)
+  int jplane;          // Jones plane (beam models)
   int expo;            // float offset of the segment's exponent tables (TcExpo), spectra and tapers
   float lam0, xi0;        // log-frequency term and squared frequency ratio at the reference channel
 };
@@ -68,7 +70,9 @@ struct TcParams {
 
 struct TcPlan {
   bool on = false;
+  bool beam = false;
   int MA = 2, NJ = 2, T = 1;  // 16 MA rows x 8 NJ columns per warp, T warps per team
+  int NC = 2;                 // column groups that are channels: NJ, or 1 for a beam (NJ correlations)
   int kind = kPoint;        // family of the (remaining) table: Point, PointSpec, Gauss, GaussSpec
   int mixed = 0;            // a point sub-table precedes the Gaussian rows (as ModelDesc.ncompPt)
   bool crossPt = false;     // point rows with a spectral index need the cross product
@@ -85,12 +89,28 @@ struct TcPlan {
 // teams and tables.  table: host copy of the table the kernels read (ncompPt
 // point rows first when mixed), rows of comp_stride floats.  Leaves plan->on
 // false (and returns) when the recurrence kernels should run.
-void tc_plan_layout(const LayoutDesc& L, const ModelDesc& M, const Plan& recur, const float* table, TcPlan* plan);
+// jchan (beam models): Jones plane per frequency-table index, ncorr modelled
+// correlations; runs never span a change of plane, and recurCost is what the
+// other form costs in the shapes' units.
+void tc_plan_layout(const LayoutDesc& L, const ModelDesc& M, const float* table, double recurCost, TcPlan* plan,
+                    const int* jchan = nullptr, int ncorr = 0);
+// Cost of the recurrence kernels for a plan of theirs.
+double tc_recur_cost(const Plan& recur);
 
 // Device side and launch.
-int tc_finalize(TcPlan* plan, const KParams& base, std::string* err);
+int tc_finalize(TcPlan* plan, const KParams& base, std::string* err);  // plan->beam: the beam kernel
 void tc_free(TcPlan* plan);
-int tc_launch(const TcPlan& plan, const Plan& recur, float* d_vis, int nvis, const float* d_comps, int* d_err,
+struct TcBeamParams {
+  TcParams t;
+  BeamKParams b;    // antenna types, Jones table, application
+  const int* perm;  // component's index in the Jones table, or null
+};
+// The beam form's kernel for the plan (dft_tc_beam.cu): resident CTAs, launch.
+int tc_beam_prepare(const TcPlan& plan, int* gridCap, std::string* err);
+int tc_beam_launch(const TcPlan& plan, const ModelDesc& model, const BeamKParams& beam, const int* perm,
+                   const float* d_comps, cudaStream_t stream, std::string* err);
+
+int tc_launch(const TcPlan& plan, const ModelDesc& model, float* d_vis, int nvis, const float* d_comps, int* d_err,
               cudaStream_t stream, std::string* err);
 
 }  // namespace obit

@@ -4,6 +4,7 @@
 // recurrence kernels.  Plain C++, no CUDA calls.
 #include <algorithm>
 #include <cmath>
+#include <iterator>
 
 #include "dft_tc.h"
 
@@ -24,6 +25,7 @@ struct Run {
   double f0, df;  // frequency ratios f0 + k df
   int list0, n;   // channel-list range
   double lnShift; // log-frequency term = ln f + lnShift
+  int jplane;
 };
 
 void split_ds(double x, float* hi, float* lo) {
@@ -40,6 +42,9 @@ struct Shape {
   int MA, NJ, T;
   double cost;
 };
+// A beam's column groups are its correlations (4 or 2).
+constexpr Shape kBeamShapes4[] = {{2, 4, 1, 700.0}, {1, 4, 1, 420.0}};
+constexpr Shape kBeamShapes2[] = {{2, 2, 1, 420.0}};
 constexpr Shape kShapes[] = {{2, 2, 2, 792.0}, {2, 2, 1, 416.0}, {1, 2, 1, 261.0}, {1, 1, 1, 192.0}};
 constexpr double kRecurCost = 1.9;
 
@@ -65,8 +70,14 @@ double max_abs(const float* table, int stride, int field, int ncomp) {
 
 }  // namespace
 
-void tc_plan_layout(const LayoutDesc& L, const ModelDesc& M, const Plan& recur, const float* table, TcPlan* plan) {
+double tc_recur_cost(const Plan& recur) {
+  return kRecurCost * recur.kp.nblocks * recur.tune.K;  // its blocks are padded too
+}
+
+void tc_plan_layout(const LayoutDesc& L, const ModelDesc& M, const float* table, double recurCost, TcPlan* plan,
+                    const int* jchan, int ncorr) {
   *plan = TcPlan();
+  const bool beam = jchan != nullptr;
   const bool spec = spec_kind(M.kind), gauss = gauss_kind(M.kind);
   if (!(M.kind == kPoint || M.kind == kGauss || (spec && M.nterm == 1))) return;
   const int npt = M.ncompPt, ntot = npt + M.ncomp;
@@ -88,11 +99,13 @@ void tc_plan_layout(const LayoutDesc& L, const ModelDesc& M, const Plan& recur, 
   std::vector<double> f;
   std::vector<int> off;
   std::vector<double> ln;
+  std::vector<int> jp;
   for (int iIF = L.ifb; iIF <= L.ife; iIF++)
     for (int ch = L.chanb; ch <= L.chane; ch++) {
       const int i = ch * L.kincf + iIF * L.kincif;
       f.push_back(L.fscale[i]);
-      off.push_back(L.nrparm + iIF * L.incif + ch * L.incf + L.stokb * L.incs);
+      off.push_back(L.nrparm + iIF * L.incif + ch * L.incf + (beam ? 0 : L.stokb * L.incs));
+      jp.push_back(beam ? jchan[i] : 0);
       ln.push_back(spec ? L.lnspec[i] : 0.0);
       if (!(L.fscale[i] > 0.0)) return;
     }
@@ -100,13 +113,13 @@ void tc_plan_layout(const LayoutDesc& L, const ModelDesc& M, const Plan& recur, 
   for (int i = 0; i < n;) {
     int e = i + 1;
     double df = 0.0;
-    if (e < n) {
+    if (e < n && jp[e] == jp[i]) {
       df = f[e] - f[i];
       // the increment's own rounding grows with the run; the run is checked
       // against its mean increment below
-      while (e < n && std::fabs(f[e] - (f[i] + (e - i) * df)) <= (1e-13 + 4.5e-16 * (e - i)) * f[i]) e++;
+      while (e < n && jp[e] == jp[i] && std::fabs(f[e] - (f[i] + (e - i) * df)) <= (1e-13 + 4.5e-16 * (e - i)) * f[i]) e++;
     }
-    Run r{f[i], df, i, e - i, spec ? ln[i] - std::log(f[i]) : 0.0};
+    Run r{f[i], df, i, e - i, spec ? ln[i] - std::log(f[i]) : 0.0, jp[i]};
     if (r.n > 1) r.df = (f[e - 1] - f[i]) / (r.n - 1);
     for (int k = 0; k < r.n; k++) {
       if (std::fabs(f[i + k] - (r.f0 + k * r.df)) > 2e-13 * f[i]) return;
@@ -125,22 +138,29 @@ void tc_plan_layout(const LayoutDesc& L, const ModelDesc& M, const Plan& recur, 
   if (!gauss && spec) amax = max_abs(table, stride, kSpecIndexField, M.ncomp);
   if (gauss && npt) amax = max_abs(table, stride, kSpecIndexField, npt);
   if (gauss && spec) amax = std::max(amax, max_abs(gt, stride, 7, M.ncomp));
-  double best = kRecurCost * recur.kp.nblocks * recur.tune.K;  // its blocks are padded too
+  double best = recurCost;
   TcPlan chosen;
-  for (const Shape& s : kShapes) {
+  std::vector<Shape> shapes;
+  if (!beam) shapes.assign(std::begin(kShapes), std::end(kShapes));
+  else if (ncorr > 2) shapes.assign(std::begin(kBeamShapes4), std::end(kBeamShapes4));
+  else shapes.assign(std::begin(kBeamShapes2), std::end(kBeamShapes2));
+  for (const Shape& s : shapes) {
     double cost = 0.0;
-    const int segCap = 128 * s.MA * s.NJ, cap = segCap * s.T;
+    const int NC = beam ? 1 : s.NJ;
+    const int segCap = 128 * s.MA * NC, cap = segCap * s.T;
     for (const Run& r : runs) cost += s.cost * ((r.n + cap - 1) / cap);
     if (!(cost < best)) continue;
     TcPlan p;
     p.MA = s.MA;
     p.NJ = s.NJ;
     p.T = s.T;
+    p.NC = NC;
+    p.beam = beam;
     p.kind = M.kind;
     p.mixed = npt > 0;
     p.chanOff = off;
-    const TcExpo lay = tc_expo_layout(s.MA, s.NJ);
-    const int D = 8 * s.NJ, a0 = 8 * (s.MA - 1) + 4, rows = 16 * s.MA, cols = 8 * s.NJ;
+    const TcExpo lay = tc_expo_layout(s.MA, NC);
+    const int D = 8 * NC, a0 = 8 * (s.MA - 1) + 4, rows = 16 * s.MA, cols = 8 * NC;
     const double inv2pi = 0.15915494309189533577;
     bool ok = true;
     double resid1 = 0.0, resid2 = 0.0, gcross = 0.0, range = 0.0;
@@ -158,6 +178,7 @@ void tc_plan_layout(const LayoutDesc& L, const ModelDesc& M, const Plan& recur, 
           g.end = r.list0 + std::min(r.n, k0 + segCap);
           split_ds(F(D * a0 + 4) * inv2pi, &g.fa_hi, &g.fa_lo);
           g.ch0 = r.list0 + k0;
+          g.jplane = r.jplane;
           if (!(spec || gauss) || k0 >= r.n) continue;
           if (!(std::min(F(0), F(segCap - 1)) > 0.05 * r.f0)) {
             ok = false;
@@ -195,7 +216,7 @@ void tc_plan_layout(const LayoutDesc& L, const ModelDesc& M, const Plan& recur, 
               // fragment order: lane (row % 8) * 4 + (column % 8) / 2
               const int mi = a >> 4, e = 2 * ((a >> 3) & 1) + (c & 1);
               const int lane = 4 * (a & 7) + ((c & 7) >> 1);
-              ex[lay.L + ((mi * s.NJ + (c >> 3)) * 32 + lane) * 4 + e] = (float)(Lg(a, c) - lam0);
+              ex[lay.L + ((mi * NC + (c >> 3)) * 32 + lane) * 4 + e] = (float)(Lg(a, c) - lam0);
             }
             const double xl = (spec && yy > 0.0) ? ry / yy : 0.0;
             ex[lay.xl + a] = (float)xl;

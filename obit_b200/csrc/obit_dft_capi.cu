@@ -57,13 +57,15 @@ struct BeamState {
   BeamSeg* d_segs = nullptr;      // channel runs of the tensor-core form
   float4* d_coef = nullptr;       // its coefficient fragments (written per launch)
   float2* d_amp = nullptr;        // its spectral amplitudes (written per launch)
+  int* d_perm = nullptr;          // Jones-table index of each row of the run table
   BeamKParams kp{};
 };
 
 void free_beam_tables(BeamState& b) {
   for (void* q : {(void*)b.d_fscale, (void*)b.d_lnspec, (void*)b.d_plane, (void*)b.d_blocks, (void*)b.d_segs,
-                  (void*)b.d_coef, (void*)b.d_amp})
+                  (void*)b.d_coef, (void*)b.d_amp, (void*)b.d_perm})
     if (q) cudaFree(q);
+  b.d_perm = nullptr;
   b.d_coef = nullptr;
   b.d_amp = nullptr;
   b.d_fscale = nullptr;
@@ -106,6 +108,10 @@ std::vector<BeamSeg> beam_segments(const Plan& plan, const LayoutDesc& L, const 
   }
   return segs;
 }
+
+// Cost of the one-phasor-per-channel tensor-core form (dft_beam_mma.cu) per
+// channel, in the units of the outer-product form's shapes (1.08 T evaluations/s).
+constexpr double kBeamMmaCost = 8.1;
 
 struct State {
   int device = 0;
@@ -196,10 +202,11 @@ void release_state(State* s) {
 //    the Gaussian components.  *md becomes that point family when no Gaussian
 //    is left, else a mixed model (md->ncompPt point rows, md->ncomp Gaussian).
 // The Gaussian rows are ordered by index too.  *index receives the ordered
-// spectral indices of the point rows, *table the copy's rows on the host; both
-// left empty (no copy made, *md unchanged) when an index is not finite or no
+// spectral indices of the point rows, *table the copy's rows on the host and
+// *order the caller's index of each row; all left empty (no copy made, *md unchanged) when an index is not finite or no
 // component qualifies.
-int prepare_run_table(State* s, ModelDesc* md, std::vector<float>* index, std::vector<float>* table) {
+int prepare_run_table(State* s, ModelDesc* md, std::vector<float>* index, std::vector<float>* table,
+                      std::vector<int>* order) {
   index->clear();
   const bool gauss = md->kind == kGaussSpec || md->kind == kGaussTSpec;
   const size_t stride = (size_t)comp_stride(*md), n = (size_t)md->ncomp;
@@ -273,6 +280,8 @@ int prepare_run_table(State* s, ModelDesc* md, std::vector<float>* index, std::v
     }
   }
   *table = std::move(out);
+  *order = std::move(pts);
+  order->insert(order->end(), gs.begin(), gs.end());
   return OBIT_DFT_OK;
 }
 
@@ -294,13 +303,14 @@ int ensure_plan(GPUInfo* g, State* s) {
   if (s->waitPolls != kDefaultWaitPolls) T.specFactor = 0;
   ModelDesc md = s->mc.model;
   std::vector<float> index, table;
+  std::vector<int> order;
   s->runComps = s->d_comps;
   const float* runLo = s->haveLo ? s->d_lo : nullptr;
   const bool ptOne = md.kind == kPointTSpec || (md.kind == kPointSpec && md.nterm == 1);
   const bool gsOne = md.kind == kGaussTSpec || (md.kind == kGaussSpec && md.nterm == 1);
   if (T.flavor == kFlavorRecur && T.specFactor && md.ncomp > 1 && (ptOne || (gsOne && !s->haveLo))) {
     ModelDesc m2 = md;
-    if ((rc = prepare_run_table(s, &m2, &index, &table))) return rc;
+    if ((rc = prepare_run_table(s, &m2, &index, &table, &order))) return rc;
     if (!index.empty()) {
       m2.specIndex = index.data();
       Plan trial;
@@ -326,7 +336,7 @@ int ensure_plan(GPUInfo* g, State* s) {
       table.resize((size_t)md.ncomp * comp_stride(md));
       CUDA_TRY(cudaMemcpy(table.data(), s->d_comps, sizeof(float) * table.size(), cudaMemcpyDeviceToHost));
     }
-    tc_plan_layout(L, md, s->plan, table.data(), &s->tc);
+    tc_plan_layout(L, md, table.data(), tc_recur_cost(s->plan), &s->tc);
     if (s->tc.on && (rc = tc_finalize(&s->tc, s->plan.kp, &err))) return fail(rc, err);
   }
   if (s->beam.on) {  // launch parameters and per-(channel, IF) tables of the beam kernel
@@ -347,7 +357,9 @@ int ensure_plan(GPUInfo* g, State* s) {
     if ((int)L.specIndex.size() >= nfreq &&
         (rc = upload(L.specIndex.data(), sizeof(int) * nfreq, (void**)&b.d_plane)))
       return rc;
-    // Channel blocks that never span a change of Jones plane, from the same
+    // The outer-product tensor-core form (dft_tc_beam.cu), where it takes the
+    // layout and model, in the run table's order; else
+    // channel blocks that never span a change of Jones plane, from the same
     // planner: 16-channel blocks joined into runs for the tensor-core form
     // (uniformly spaced channels, runs of 4 channels or more
     // on average), else blocks of at most kBeamK channels for the block form.
@@ -360,7 +372,22 @@ int ensure_plan(GPUInfo* g, State* s) {
     Plan mplan, bplan;
     std::vector<BeamSeg> segs;
     bool mma = false;
-    if (s->tune.flavor == kFlavorRecur && s->tune.specFactor && beam_mma_supported(s->mc.model.kind)) {
+    if (T.flavor == kFlavorRecur && T.specFactor && T.K == 0 && T.ct == 0 && T.Bt == 0 && T.threads == 0 &&
+        s->plan.linear && md.ncompPt + md.ncomp >= kTcMinComps) {
+      if (s->runComps == s->d_comps) {
+        table.resize((size_t)md.ncomp * comp_stride(md));
+        CUDA_TRY(cudaMemcpy(table.data(), s->d_comps, sizeof(float) * table.size(), cudaMemcpyDeviceToHost));
+      }
+      const int ncorr = L.nstok >= 4 ? 4 : std::min(2, L.nstok);
+      long long nch = (long long)(L.chane - L.chanb + 1) * (L.ife - L.ifb + 1);
+      tc_plan_layout(L, md, table.data(), kBeamMmaCost * (double)nch, &s->tc, b.jchan.data(), ncorr);
+      if (s->tc.on) {
+        if ((rc = tc_finalize(&s->tc, s->plan.kp, &err))) return fail(rc, err);
+        if (s->runComps == s->d_sorted && (rc = upload(order.data(), sizeof(int) * order.size(), (void**)&b.d_perm)))
+          return rc;
+      }
+    }
+    if (!s->tc.on && s->tune.flavor == kFlavorRecur && s->tune.specFactor && beam_mma_supported(s->mc.model.kind)) {
       TB.K = kBeamMmaRows;
       rc = plan_layout(LB, s->mc.model, A, TB, &mplan, &err);
       if (rc) return fail(rc, err);
@@ -385,7 +412,7 @@ int ensure_plan(GPUInfo* g, State* s) {
         }
       }
     }
-    if (!mma) {
+    if (!mma) {  // (also the fields that the outer-product form shares)
       TB.K = kBeamK;
       rc = plan_layout(LB, s->mc.model, A, TB, &bplan, &err);
       if (rc) return fail(rc, err);
@@ -457,7 +484,7 @@ int ensure_plan(GPUInfo* g, State* s) {
         CUDA_TRY(cudaMalloc(&b.d_amp, ab));
         k.ampTab = b.d_amp;
       }
-    } else if ((rc = beam_fit_tile(&k, &err))) {
+    } else if (!s->tc.on && (rc = beam_fit_tile(&k, &err))) {
       return fail(rc, err);
     }
   }
@@ -465,9 +492,19 @@ int ensure_plan(GPUInfo* g, State* s) {
   return OBIT_DFT_OK;
 }
 
+// The beam-corrected model over nvis records at d_vis; prologue: write the
+// tables of the forms that have them.
+int launch_beam_model(State* s, float* d_vis, int nvis, cudaStream_t stream, std::string* err, bool prologue) {
+  BeamKParams k = s->beam.kp;
+  k.k.vis = d_vis;
+  k.k.nvis = nvis;
+  if (s->tc.on) return tc_beam_launch(s->tc, s->plan.model, k, s->beam.d_perm, s->runComps, stream, err);
+  return launch_beam(k, stream, err, prologue);
+}
+
 // The plain sky model over nvis records at d_vis.
 int launch_model(State* s, float* d_vis, int nvis, cudaStream_t stream, std::string* err) {
-  if (s->tc.on) return tc_launch(s->tc, s->plan, d_vis, nvis, s->runComps, s->d_err, stream, err);
+  if (s->tc.on) return tc_launch(s->tc, s->plan.model, d_vis, nvis, s->runComps, s->d_err, stream, err);
   return launch_plan(s->plan, d_vis, 0, nvis, s->runComps, s->d_err, stream, err);
 }
 
@@ -728,10 +765,7 @@ int obit_dft_calc_device(GPUInfo* g, float* d_vis, int nvis, void* stream) {
   if (rc) return rc;
   std::string err;
   if (s->beam.on) {
-    BeamKParams k = s->beam.kp;
-    k.k.vis = d_vis;
-    k.k.nvis = nvis;
-    rc = launch_beam(k, (cudaStream_t)stream, &err);
+    rc = launch_beam_model(s, d_vis, nvis, (cudaStream_t)stream, &err, true);
   } else {
     rc = launch_model(s, d_vis, nvis, (cudaStream_t)stream, &err);
   }
@@ -765,7 +799,9 @@ int obit_dft_beam_info(GPUInfo* g, int* info, int n) {
   rc = ensure_plan(g, s);
   if (rc) return rc;
   const BeamKParams& k = s->beam.kp;
-  const int v[3] = {k.mma ? 1 : (k.flavor == kFlavorPlain ? 2 : 0), k.k.ct, k.mma ? k.nseg : k.k.nblocks};
+  const bool outer = s->tc.on;
+  const int v[3] = {outer || k.mma ? 1 : (k.flavor == kFlavorPlain ? 2 : 0), outer ? kTcChunk : k.k.ct,
+                    outer ? (int)s->tc.teams.size() : k.mma ? k.nseg : k.k.nblocks};
   for (int i = 0; i < n && i < 3; i++) info[i] = v[i];
   return OBIT_DFT_OK;
 }
@@ -857,10 +893,7 @@ int obit_dft_calc(GPUInfo* g) {
     float* host = g->h_data + (size_t)r0 * lenvis;
     CUDA_TRY(cudaMemcpyAsync(bufs[b], host, bytes, cudaMemcpyHostToDevice, streams[b]));
     if (s->beam.on) {
-      BeamKParams k = s->beam.kp;
-      k.k.vis = bufs[b];
-      k.k.nvis = nr;
-      rc = launch_beam(k, streams[b], &err, !beamPrologue);
+      rc = launch_beam_model(s, bufs[b], nr, streams[b], &err, !beamPrologue);
     } else {
       rc = launch_model(s, bufs[b], nr, streams[b], &err);
     }

@@ -19,6 +19,7 @@
 
 #include "abi_internal.h"
 #include "dft_plan.h"
+#include "dft_tc.h"
 #include "obit_dft.h"
 
 using namespace obit;
@@ -47,6 +48,9 @@ struct Facet {
   int nvis = 0;
   size_t compOff = 0;        // float offset in the batch's padded component buffer
   long long evalsPerRow = 0; // selected (channel, IF) pairs x components
+  // the tensor-core form's launches, where it takes the facet (else its group's
+  // persistent kernel does)
+  std::vector<TcPlan> tc;
   // planner-default single-facet plans for the per-facet comparator
   Plan single[2];
   bool haveSingle[2] = {false, false};
@@ -62,6 +66,7 @@ struct Group {
   size_t smemBytes = 0;
   int cap = 0;                // CTAs resident across the device
   long long items = 0, evals = 0;
+  long long listed = 0;       // items with those the tensor-core form took
   std::vector<KParams> hkps;  // host copies of the facets' parameter blocks (group order)
   KParams* d_params = nullptr;
   int* d_itemStart = nullptr;
@@ -117,6 +122,12 @@ struct ObitDFTBatch {
   int* d_err = nullptr;
   std::vector<Group> groups;
   cudaStream_t capStream = nullptr;
+  bool tileSet = false;  // obit_dft_batch_set_tile asked for a recurrence tile
+  // branches of the captured graphs that hold the tensor-core launches, and
+  // their fork and join events
+  static constexpr int kBranches = 8;
+  cudaStream_t branch[kBranches] = {};
+  cudaEvent_t branchEv[kBranches + 1] = {};
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   HostRun host;
@@ -133,9 +144,12 @@ void drop_graph(ObitDFTBatch* b) {
 }
 
 // Plan every facet of group g with one tile shape and upload its work list.
-// Facets are read from `fs` (the batch's own, or a row sample's).
-int build_group(Group& g, std::vector<Facet>& fs, const float* d_comps, int* d_err, std::string* err) {
+// Facets are read from `fs` (the batch's own, or a row sample's).  tensor: those
+// that the tensor-core form takes are left out of the launched work list.
+int build_group(Group& g, std::vector<Facet>& fs, const float* d_comps, int* d_err, std::string* err,
+                bool tensor = false) {
   free_group(g);
+  g.listed = 0;
   if (g.order.empty()) return 0;
   // the tile shape: requested fields, else the planner's choice for the
   // facet of the most work
@@ -195,6 +209,8 @@ int build_group(Group& g, std::vector<Facet>& fs, const float* d_comps, int* d_e
     long long n = 0;
     if (fs[f].nvis > 0 && fs[f].mc.model.ncomp > 0 && p.kp.nblocks > 0)
       n = (long long)((fs[f].nvis + p.kp.R - 1) / p.kp.R) * p.kp.nBlockTiles;
+    g.listed += n;
+    if (tensor && !fs[f].tc.empty()) n = 0;
     items += n;
     if (items > (long long)INT32_MAX - 1) {
       *err = "batch has more than 2^31 work items";
@@ -239,7 +255,7 @@ int build_group(Group& g, std::vector<Facet>& fs, const float* d_comps, int* d_e
   g.cap = cap;
   g.items = items;
   g.evals = evals;
-  g.grid = (int)std::min<long long>(items, cap);
+  g.grid = (int)std::min<long long>(items, cap);  // (0: nothing left to launch)
   g.built = true;
   return 0;
 }
@@ -263,10 +279,51 @@ int ensure_built(ObitDFTBatch* b) {
   std::string err;
   for (Group& g : b->groups)
     if (!g.built) {
-      int rc = build_group(g, b->facets, b->d_comps, b->d_err, &err);
+      int rc = build_group(g, b->facets, b->d_comps, b->d_err, &err, !b->tileSet);
       if (rc) return fail(rc, err);
     }
   return 0;
+}
+
+// Tensor-core launches of pieces of facets inside a capture on cs: the most
+// work first, spread over branches of the graph so that small facets' launches
+// overlap, beside what `rest` captures on cs.  (Bitwise the same for any cut of the rows: records are independent.)
+struct TcPiece {
+  int f;
+  float* d_vis;
+  int nvis;
+};
+template <class Rest>
+int capture_tensor(ObitDFTBatch* b, cudaStream_t cs, std::vector<TcPiece> ps, std::string* err, Rest rest) {
+  ps.erase(std::remove_if(ps.begin(), ps.end(), [&](const TcPiece& p) { return b->facets[p.f].tc.empty() || p.nvis <= 0; }),
+           ps.end());
+  if (b->tileSet || ps.empty()) return rest();
+  auto cost = [&](const TcPiece& p) { return (double)p.nvis * (double)b->facets[p.f].evalsPerRow; };
+  std::stable_sort(ps.begin(), ps.end(), [&](const TcPiece& x, const TcPiece& y) { return cost(x) > cost(y); });
+  const int nb = std::min<int>(ObitDFTBatch::kBranches, (int)ps.size());
+  cudaError_t ce = cudaEventRecord(b->branchEv[ObitDFTBatch::kBranches], cs);
+  for (int i = 0; i < nb && ce == cudaSuccess; i++) ce = cudaStreamWaitEvent(b->branch[i], b->branchEv[ObitDFTBatch::kBranches], 0);
+  std::vector<double> load(nb, 0.0);
+  int rc = 0;
+  for (const TcPiece& p : ps) {
+    if (rc || ce != cudaSuccess) break;
+    const int at = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+    load[at] += cost(p);
+    const Facet& f = b->facets[p.f];
+    for (const TcPlan& part : f.tc)
+      if (!rc) rc = tc_launch(part, f.mc.model, p.d_vis, p.nvis, b->d_comps + f.compOff, b->d_err, b->branch[at], err);
+  }
+  if (!rc && ce == cudaSuccess) rc = rest();
+  for (int i = 0; i < nb; i++) {  // join even after a failure, so that the capture can end
+    const cudaError_t c1 = cudaEventRecord(b->branchEv[i], b->branch[i]);
+    const cudaError_t c2 = c1 == cudaSuccess ? cudaStreamWaitEvent(cs, b->branchEv[i], 0) : c1;
+    if (ce == cudaSuccess) ce = c2;
+  }
+  if (!rc && ce != cudaSuccess) {
+    *err = std::string("tensor-core branches: ") + cudaGetErrorString(ce);
+    rc = OBIT_DFT_ECUDA;
+  }
+  return rc;
 }
 
 const Group* main_group(const ObitDFTBatch* b) {
@@ -346,7 +403,8 @@ int build_host_run(ObitDFTBatch* b, float* const* h, long long stagingBytes) {
         kp.vis = r.d_stage + (w % 2) * half + pc.off;
         kp.nvis = pc.n;
         kp.rowBase = 0;
-        if (kp.ncomp > 0 && kp.nblocks > 0) L.items += (long long)((pc.n + kp.R - 1) / kp.R) * kp.nBlockTiles;
+        const bool tensor = !b->tileSet && !b->facets[pc.f].tc.empty();
+        if (kp.ncomp > 0 && kp.nblocks > 0 && !tensor) L.items += (long long)((pc.n + kp.R - 1) / kp.R) * kp.nBlockTiles;
         kps.push_back(kp);
         starts.push_back((int)L.items);
       }
@@ -399,19 +457,26 @@ int build_host_run(ObitDFTBatch* b, float* const* h, long long stagingBytes) {
     if (ce == cudaSuccess) ce = copy_wave(w, true);
     if (ce == cudaSuccess) ce = cudaEventRecord(up(w), cp);
     if (ce == cudaSuccess) ce = cudaStreamWaitEvent(cs, up(w), 0);
-    for (; li < launches.size() && launches[li].wave == w && ce == cudaSuccess && !rc; li++) {
-      const Launch& L = launches[li];
-      const Group& g = b->groups[L.group];
-      if (L.items <= 0) continue;
-      ce = cudaMemsetAsync(r.d_counters + li, 0, sizeof(int), cs);
-      if (ce != cudaSuccess) break;
-      BatchParams bp{};
-      bp.facets = r.d_params + L.params;
-      bp.itemStart = r.d_starts + L.start;
-      bp.nfacet = (int)L.pieces;
-      bp.counter = r.d_counters + li;
-      rc = launch_batch(g.K, g.kind, bp, (int)std::min<long long>(L.items, g.cap), g.threads, g.smemBytes, cs, &err);
-    }
+    std::vector<TcPiece> ps;
+    for (const Piece& pc : waves[w]) ps.push_back({pc.f, r.d_stage + (w % 2) * half + pc.off, pc.n});
+    if (ce == cudaSuccess)
+      rc = capture_tensor(b, cs, ps, &err, [&]() {
+        int rg = 0;
+        for (; li < launches.size() && launches[li].wave == w && ce == cudaSuccess && !rg; li++) {
+          const Launch& L = launches[li];
+          const Group& g = b->groups[L.group];
+          if (L.items <= 0) continue;
+          ce = cudaMemsetAsync(r.d_counters + li, 0, sizeof(int), cs);
+          if (ce != cudaSuccess) break;
+          BatchParams bp{};
+          bp.facets = r.d_params + L.params;
+          bp.itemStart = r.d_starts + L.start;
+          bp.nfacet = (int)L.pieces;
+          bp.counter = r.d_counters + li;
+          rg = launch_batch(g.K, g.kind, bp, (int)std::min<long long>(L.items, g.cap), g.threads, g.smemBytes, cs, &err);
+        }
+        return rg;
+      });
     if (ce == cudaSuccess) ce = cudaEventRecord(done(w), cs);
   }
   for (size_t w = (nw >= 2 ? nw - 2 : 0); w < nw && ce == cudaSuccess; w++) {
@@ -504,6 +569,22 @@ extern "C" int obit_dft_batch_create(const ObitDFTFacet* in, int nfacet, ObitDFT
     it->order.push_back(i);
   }
   CUDA_TRY(cudaStreamCreateWithFlags(&b->capStream, cudaStreamNonBlocking));
+  for (cudaStream_t& st : b->branch) CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+  for (cudaEvent_t& ev : b->branchEv) CUDA_TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+  // the tensor-core form of each facet, in the caller's component order
+  for (Facet& f : b->facets) {
+    const ModelDesc& md = f.mc.model;
+    if (md.ncomp < kTcMinComps || f.nvis <= 0) continue;
+    Plan p;
+    if (plan_layout(f.L, md, f.A, TuneDesc(), &p, &err) || !p.linear) continue;
+    std::vector<float> table((size_t)md.ncomp * comp_stride(md));
+    CUDA_TRY(cudaMemcpy(table.data(), b->d_comps + f.compOff, sizeof(float) * table.size(), cudaMemcpyDeviceToHost));
+    tc_plan_layout(f.L, md, table.data(), tc_recur_cost(p), &f.tc);
+    if (int rc = tc_finalize_all(&f.tc, p.kp, &err)) {
+      obit_dft_batch_destroy(b.release());
+      return fail(rc, err);
+    }
+  }
   int rc = ensure_built(b.get());
   if (rc) {
     obit_dft_batch_destroy(b.release());
@@ -522,6 +603,7 @@ extern "C" int obit_dft_batch_set_tile(ObitDFTBatch* b, int K, int ct, int Bt, i
   CUDA_TRY(cudaSetDevice(b->device));
   CUDA_TRY(cudaDeviceSynchronize());
   drop_graph(b);
+  b->tileSet = K || ct || Bt || threads;
   for (Group& g : b->groups) {
     g.tune.K = K;
     g.tune.ct = ct ? ct : 128;
@@ -541,10 +623,14 @@ extern "C" int obit_dft_batch_run(ObitDFTBatch* b, void* stream) {
   if (!b->exec) {
     std::string err;
     CUDA_TRY(cudaStreamBeginCapture(b->capStream, cudaStreamCaptureModeThreadLocal));
-    for (const Group& g : b->groups) {
-      rc = launch_group(g, b->capStream, &err);
-      if (rc) break;
-    }
+    std::vector<TcPiece> ps;
+    for (size_t f = 0; f < b->facets.size(); f++) ps.push_back({(int)f, b->facets[f].d_vis, b->facets[f].nvis});
+    rc = capture_tensor(b, b->capStream, ps, &err, [&]() {
+      int rg = 0;
+      for (const Group& g : b->groups)
+        if ((rg = launch_group(g, b->capStream, &err))) break;
+      return rg;
+    });
     cudaGraph_t graph = nullptr;
     cudaError_t ce = cudaStreamEndCapture(b->capStream, &graph);
     if (rc) {
@@ -785,9 +871,9 @@ extern "C" int obit_dft_batch_info(ObitDFTBatch* b, long long* info, int n) {
   if (!b || (!info && n > 0)) return fail(OBIT_DFT_EBADARG, "NULL argument");
   long long items = 0, evals = 0, launches = 0;
   for (const Group& g : b->groups) {
-    items += g.items;
+    items += g.listed;
     evals += g.evals;
-    launches += g.items > 0;
+    launches += g.listed > 0;
   }
   const Group* m = main_group(b);
   const long long v[10] = {(long long)b->facets.size(), launches, items, evals,
@@ -804,9 +890,15 @@ extern "C" int obit_dft_batch_destroy(ObitDFTBatch* b) {
   cudaDeviceSynchronize();
   drop_graph(b);
   for (Group& g : b->groups) free_group(g);
-  for (Facet& f : b->facets)
+  for (Facet& f : b->facets) {
     for (int k = 0; k < 2; k++)
       if (f.haveSingle[k]) free_plan(&f.single[k]);
+    tc_free(&f.tc);
+  }
+  for (cudaStream_t st : b->branch)
+    if (st) cudaStreamDestroy(st);
+  for (cudaEvent_t ev : b->branchEv)
+    if (ev) cudaEventDestroy(ev);
   if (b->d_comps) cudaFree(b->d_comps);
   if (b->d_err) cudaFree(b->d_err);
   if (b->capStream) cudaStreamDestroy(b->capStream);

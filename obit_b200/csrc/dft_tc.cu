@@ -130,9 +130,16 @@ int tc_finalize(TcPlan* plan, const KParams& base, std::string* err) {
   return 0;
 }
 
-void tc_free(TcPlan* plan) {
-  if (plan->d_mem) cudaFree(plan->d_mem);
-  *plan = TcPlan();
+int tc_finalize_all(std::vector<TcPlan>* plan, const KParams& base, std::string* err) {
+  for (TcPlan& p : *plan)
+    if (int rc = tc_finalize(&p, base, err)) return rc;
+  return 0;
+}
+
+void tc_free(std::vector<TcPlan>* plan) {
+  for (TcPlan& p : *plan)
+    if (p.d_mem) cudaFree(p.d_mem);
+  plan->clear();
 }
 
 int tc_launch(const TcPlan& plan, const ModelDesc& model, float* d_vis, int nvis, const float* d_comps, int* d_err,

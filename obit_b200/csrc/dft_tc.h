@@ -68,6 +68,8 @@ struct TcParams {
   int specField;            // component field of the spectral index
 };
 
+// One launch: teams of one shape.  A model's plan is one of these per shape that
+// its runs are cut into.
 struct TcPlan {
   bool on = false;
   bool beam = false;
@@ -87,19 +89,20 @@ struct TcPlan {
 
 // Host part: whether the tensor-core form takes this layout and model, and its
 // teams and tables.  table: host copy of the table the kernels read (ncompPt
-// point rows first when mixed), rows of comp_stride floats.  Leaves plan->on
-// false (and returns) when the recurrence kernels should run.
+// point rows first when mixed), rows of comp_stride floats.  Leaves *plan
+// empty when the recurrence kernels should run.
 // jchan (beam models): Jones plane per frequency-table index, ncorr modelled
 // correlations; runs never span a change of plane, and recurCost is what the
 // other form costs in the shapes' units.
-void tc_plan_layout(const LayoutDesc& L, const ModelDesc& M, const float* table, double recurCost, TcPlan* plan,
-                    const int* jchan = nullptr, int ncorr = 0);
+void tc_plan_layout(const LayoutDesc& L, const ModelDesc& M, const float* table, double recurCost,
+                    std::vector<TcPlan>* plan, const int* jchan = nullptr, int ncorr = 0);
 // Cost of the recurrence kernels for a plan of theirs.
 double tc_recur_cost(const Plan& recur);
 
 // Device side and launch.
 int tc_finalize(TcPlan* plan, const KParams& base, std::string* err);  // plan->beam: the beam kernel
-void tc_free(TcPlan* plan);
+void tc_free(std::vector<TcPlan>* plan);
+int tc_finalize_all(std::vector<TcPlan>* plan, const KParams& base, std::string* err);
 struct TcBeamParams {
   TcParams t;
   BeamKParams b;    // antenna types, Jones table, application

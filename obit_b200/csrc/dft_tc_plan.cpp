@@ -4,7 +4,8 @@
 // recurrence kernels.  Plain C++, no CUDA calls.
 #include <algorithm>
 #include <cmath>
-#include <iterator>
+#include <functional>
+#include <map>
 
 #include "dft_tc.h"
 
@@ -74,9 +75,9 @@ double tc_recur_cost(const Plan& recur) {
   return kRecurCost * recur.kp.nblocks * recur.tune.K;  // its blocks are padded too
 }
 
-void tc_plan_layout(const LayoutDesc& L, const ModelDesc& M, const float* table, double recurCost, TcPlan* plan,
-                    const int* jchan, int ncorr) {
-  *plan = TcPlan();
+void tc_plan_layout(const LayoutDesc& L, const ModelDesc& M, const float* table, double recurCost,
+                    std::vector<TcPlan>* plan, const int* jchan, int ncorr) {
+  plan->clear();
   const bool beam = jchan != nullptr;
   const bool spec = spec_kind(M.kind), gauss = gauss_kind(M.kind);
   if (!(M.kind == kPoint || M.kind == kGauss || (spec && M.nterm == 1))) return;
@@ -138,18 +139,21 @@ void tc_plan_layout(const LayoutDesc& L, const ModelDesc& M, const float* table,
   if (!gauss && spec) amax = max_abs(table, stride, kSpecIndexField, M.ncomp);
   if (gauss && npt) amax = max_abs(table, stride, kSpecIndexField, npt);
   if (gauss && spec) amax = std::max(amax, max_abs(gt, stride, 7, M.ncomp));
-  double best = recurCost;
-  TcPlan chosen;
   std::vector<Shape> shapes;
-  if (!beam) shapes.assign(std::begin(kShapes), std::end(kShapes));
-  else if (ncorr > 2) shapes.assign(std::begin(kBeamShapes4), std::end(kBeamShapes4));
-  else shapes.assign(std::begin(kBeamShapes2), std::end(kBeamShapes2));
-  for (const Shape& s : shapes) {
-    double cost = 0.0;
-    const int NC = beam ? 1 : s.NJ;
-    const int segCap = 128 * s.MA * NC, cap = segCap * s.T;
-    for (const Run& r : runs) cost += s.cost * ((r.n + cap - 1) / cap);
-    if (!(cost < best)) continue;
+  if (!beam)
+    for (const Shape& s : kShapes) shapes.push_back(s);
+  else if (ncorr > 2)
+    for (const Shape& s : kBeamShapes4) shapes.push_back(s);
+  else
+    for (const Shape& s : kBeamShapes2) shapes.push_back(s);
+  auto capacity = [&](const Shape& s) { return 128 * s.MA * (beam ? 1 : s.NJ) * s.T; };
+
+  // Teams of shape s over pieces of runs; false when a bound fails.
+  struct Piece {
+    int run, t0;
+  };
+  auto build = [&](const Shape& s, const std::vector<Piece>& pieces, TcPlan* out) -> bool {
+    const int NC = beam ? 1 : s.NJ, segCap = 128 * s.MA * NC;
     TcPlan p;
     p.MA = s.MA;
     p.NJ = s.NJ;
@@ -162,10 +166,11 @@ void tc_plan_layout(const LayoutDesc& L, const ModelDesc& M, const float* table,
     const TcExpo lay = tc_expo_layout(s.MA, NC);
     const int D = 8 * NC, a0 = 8 * (s.MA - 1) + 4, rows = 16 * s.MA, cols = 8 * NC;
     const double inv2pi = 0.15915494309189533577;
-    bool ok = true;
     double resid1 = 0.0, resid2 = 0.0, gcross = 0.0, range = 0.0;
-    for (const Run& r : runs) {
-      for (int t0 = 0; t0 < r.n && ok; t0 += cap) {
+    for (const Piece& pc : pieces) {
+      const Run& r = runs[pc.run];
+      const int t0 = pc.t0;
+      {
         TcTeamDesc tm{};
         tm.D = D;
         split_ds(D * r.df * inv2pi, &tm.w_hi, &tm.w_lo);
@@ -180,10 +185,7 @@ void tc_plan_layout(const LayoutDesc& L, const ModelDesc& M, const float* table,
           g.ch0 = r.list0 + k0;
           g.jplane = r.jplane;
           if (!(spec || gauss) || k0 >= r.n) continue;
-          if (!(std::min(F(0), F(segCap - 1)) > 0.05 * r.f0)) {
-            ok = false;
-            break;
-          }
+          if (!(std::min(F(0), F(segCap - 1)) > 0.05 * r.f0)) return false;
           // exponent tables: rows a against the middle column, columns n against the middle row
           g.expo = (int)p.expo.size();
           p.expo.resize(p.expo.size() + lay.total, 0.0f);
@@ -234,25 +236,67 @@ void tc_plan_layout(const LayoutDesc& L, const ModelDesc& M, const float* table,
         }
         p.teams.push_back(tm);
       }
-      if (!ok) break;
     }
-    if (!ok) continue;
     auto second = [&](double x) { return 0.5 * x * x; };
-    if (spec && amax * range > 8.0) continue;
+    if (spec && amax * range > 8.0) return false;
     if ((!gauss && spec) || npt) {
       p.crossPt = spreadPt * resid1 > kTcResidualTol || second(spreadPt * range) > kTcFirstTol;
-      if (p.crossPt && std::max(spreadPt * resid2, second(spreadPt * resid1)) > kTcResidualTol) continue;
+      if (p.crossPt && std::max(spreadPt * resid2, second(spreadPt * resid1)) > kTcResidualTol) return false;
     }
     if (gauss) {
       // second order of the taper's cross exponent q c times the taper exp(-q): largest at q = 2
-      if (0.2707 * gcross * gcross > kTcResidualTol) continue;
-      if (spec && std::max(spreadG * resid2, second(spreadG * resid1)) > kTcResidualTol) continue;
+      if (0.2707 * gcross * gcross > kTcResidualTol) return false;
+      if (spec && std::max(spreadG * resid2, second(spreadG * resid1)) > kTcResidualTol) return false;
     }
     p.on = true;
-    best = cost;
-    chosen = std::move(p);
+    *out = std::move(p);
+    return true;
+  };
+
+  // shapes that hold the bounds over whole runs, then the cheapest cover of each
+  // run by them (a run longer than a shape's capacity continues with any shape)
+  std::vector<Shape> fit;
+  for (const Shape& s : shapes) {
+    std::vector<Piece> all;
+    for (size_t i = 0; i < runs.size(); i++)
+      for (int t0 = 0; t0 < runs[i].n; t0 += capacity(s)) all.push_back({(int)i, t0});
+    TcPlan trial;
+    if (build(s, all, &trial)) fit.push_back(s);
   }
-  *plan = std::move(chosen);
+  if (fit.empty()) return;
+  std::map<int, std::pair<double, int>> cover;  // channels left -> (cost, shape)
+  cover[0] = {0.0, -1};
+  std::function<double(int)> cheapest = [&](int left) -> double {
+    auto it = cover.find(left);
+    if (it != cover.end()) return it->second.first;
+    std::pair<double, int> best{1e300, -1};
+    for (size_t i = 0; i < fit.size(); i++) {
+      const double c = fit[i].cost + cheapest(std::max(0, left - capacity(fit[i])));
+      if (c < best.first) best = {c, (int)i};
+    }
+    cover[left] = best;
+    return best.first;
+  };
+  double cost = 0.0;
+  std::vector<std::vector<Piece>> use(fit.size());
+  for (size_t i = 0; i < runs.size(); i++) {
+    if (runs[i].n > 65536) return;
+    cost += cheapest(runs[i].n);
+    for (int t0 = 0; t0 < runs[i].n;) {
+      const int k = cover[runs[i].n - t0].second;
+      use[k].push_back({(int)i, t0});
+      t0 += capacity(fit[k]);
+    }
+  }
+  if (!(cost < recurCost)) return;
+  std::vector<TcPlan> parts;
+  for (size_t k = 0; k < fit.size(); k++) {
+    if (use[k].empty()) continue;
+    TcPlan p;
+    if (!build(fit[k], use[k], &p)) return;
+    parts.push_back(std::move(p));
+  }
+  *plan = std::move(parts);
 }
 
 }  // namespace obit

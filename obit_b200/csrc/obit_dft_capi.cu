@@ -134,7 +134,7 @@ struct State {
   const float* runComps = nullptr;  // table the plan's launches read
   // plan
   Plan plan;
-  TcPlan tc;  // the tensor-core form, where it takes the plan's layout and model
+  std::vector<TcPlan> tc;  // the tensor-core form, where it takes the plan's layout and model
   bool planValid = false;
   // staging
   int bufRows = 0;                 // rows per device staging buffer
@@ -337,7 +337,7 @@ int ensure_plan(GPUInfo* g, State* s) {
       CUDA_TRY(cudaMemcpy(table.data(), s->d_comps, sizeof(float) * table.size(), cudaMemcpyDeviceToHost));
     }
     tc_plan_layout(L, md, table.data(), tc_recur_cost(s->plan), &s->tc);
-    if (s->tc.on && (rc = tc_finalize(&s->tc, s->plan.kp, &err))) return fail(rc, err);
+    if ((rc = tc_finalize_all(&s->tc, s->plan.kp, &err))) return fail(rc, err);
   }
   if (s->beam.on) {  // launch parameters and per-(channel, IF) tables of the beam kernel
     BeamState& b = s->beam;
@@ -381,13 +381,13 @@ int ensure_plan(GPUInfo* g, State* s) {
       const int ncorr = L.nstok >= 4 ? 4 : std::min(2, L.nstok);
       long long nch = (long long)(L.chane - L.chanb + 1) * (L.ife - L.ifb + 1);
       tc_plan_layout(L, md, table.data(), kBeamMmaCost * (double)nch, &s->tc, b.jchan.data(), ncorr);
-      if (s->tc.on) {
-        if ((rc = tc_finalize(&s->tc, s->plan.kp, &err))) return fail(rc, err);
+      if (!s->tc.empty()) {
+        if ((rc = tc_finalize_all(&s->tc, s->plan.kp, &err))) return fail(rc, err);
         if (s->runComps == s->d_sorted && (rc = upload(order.data(), sizeof(int) * order.size(), (void**)&b.d_perm)))
           return rc;
       }
     }
-    if (!s->tc.on && s->tune.flavor == kFlavorRecur && s->tune.specFactor && beam_mma_supported(s->mc.model.kind)) {
+    if (s->tc.empty() && s->tune.flavor == kFlavorRecur && s->tune.specFactor && beam_mma_supported(s->mc.model.kind)) {
       TB.K = kBeamMmaRows;
       rc = plan_layout(LB, s->mc.model, A, TB, &mplan, &err);
       if (rc) return fail(rc, err);
@@ -484,7 +484,7 @@ int ensure_plan(GPUInfo* g, State* s) {
         CUDA_TRY(cudaMalloc(&b.d_amp, ab));
         k.ampTab = b.d_amp;
       }
-    } else if (!s->tc.on && (rc = beam_fit_tile(&k, &err))) {
+    } else if (s->tc.empty() && (rc = beam_fit_tile(&k, &err))) {
       return fail(rc, err);
     }
   }
@@ -498,13 +498,17 @@ int launch_beam_model(State* s, float* d_vis, int nvis, cudaStream_t stream, std
   BeamKParams k = s->beam.kp;
   k.k.vis = d_vis;
   k.k.nvis = nvis;
-  if (s->tc.on) return tc_beam_launch(s->tc, s->plan.model, k, s->beam.d_perm, s->runComps, stream, err);
+  for (const TcPlan& part : s->tc)
+    if (int rc = tc_beam_launch(part, s->plan.model, k, s->beam.d_perm, s->runComps, stream, err)) return rc;
+  if (!s->tc.empty()) return 0;
   return launch_beam(k, stream, err, prologue);
 }
 
 // The plain sky model over nvis records at d_vis.
 int launch_model(State* s, float* d_vis, int nvis, cudaStream_t stream, std::string* err) {
-  if (s->tc.on) return tc_launch(s->tc, s->plan.model, d_vis, nvis, s->runComps, s->d_err, stream, err);
+  for (const TcPlan& part : s->tc)
+    if (int rc = tc_launch(part, s->plan.model, d_vis, nvis, s->runComps, s->d_err, stream, err)) return rc;
+  if (!s->tc.empty()) return 0;
   return launch_plan(s->plan, d_vis, 0, nvis, s->runComps, s->d_err, stream, err);
 }
 
@@ -784,7 +788,7 @@ int obit_dft_plan_info(GPUInfo* g, int* info, int n) {
   const Plan& pl = s->plan;
   const int v[12] = {pl.tune.flavor, pl.tune.K, pl.kp.ct, pl.kp.Bt, pl.kp.R, pl.threads,
                      pl.kp.nblocks, pl.kp.ndf, pl.specFactored ? 1 : 0, pl.mixed ? 1 : 0,
-                     pl.mixed ? pl.model.ncompPt : 0, s->tc.on ? 128 * s->tc.MA * s->tc.NJ * s->tc.T : 0};
+                     pl.mixed ? pl.model.ncompPt : 0, s->tc.empty() ? 0 : 128 * s->tc[0].MA * s->tc[0].NJ * s->tc[0].T};
   for (int i = 0; i < n && i < 12; i++) info[i] = v[i];
   return OBIT_DFT_OK;
 }
@@ -799,9 +803,11 @@ int obit_dft_beam_info(GPUInfo* g, int* info, int n) {
   rc = ensure_plan(g, s);
   if (rc) return rc;
   const BeamKParams& k = s->beam.kp;
-  const bool outer = s->tc.on;
+  const bool outer = !s->tc.empty();
+  int teams = 0;
+  for (const TcPlan& part : s->tc) teams += (int)part.teams.size();
   const int v[3] = {outer || k.mma ? 1 : (k.flavor == kFlavorPlain ? 2 : 0), outer ? kTcChunk : k.k.ct,
-                    outer ? (int)s->tc.teams.size() : k.mma ? k.nseg : k.k.nblocks};
+                    outer ? teams : k.mma ? k.nseg : k.k.nblocks};
   for (int i = 0; i < n && i < 3; i++) info[i] = v[i];
   return OBIT_DFT_OK;
 }

@@ -136,3 +136,37 @@ def test_what_it_leaves_to_the_recurrence():
     g, s5 = small(U.MOD_GAUSS, nrow=4, nchan=256, nif=1, ncomp=100)
     s5.comps[7, 4] = 1e-12
     assert _plan(g, s5)["tensorChannels"] == 0
+
+
+def test_batch_facets_on_the_tensor_cores():
+    """Facets that the tensor-core form takes (in branches of the batch's graph)
+    beside ones it does not: each against the oracle, and the streamed run over
+    host records bit for bit the same."""
+    torch = pytest.importorskip("torch")
+    from obit_b200.batch import DFTBatch, Facet
+
+    cases, facets, keep = [], [], []
+    for i, (mt, nrow, nchan, nif, ncomp) in enumerate([
+            (U.MOD_POINT, 40, 256, 1, 200), (U.MOD_POINT, 7, 130, 3, 900), (U.MOD_POINT, 33, 32, 1, 60),
+            (U.MOD_POINT_SPEC, 12, 128, 2, 75), (U.MOD_GAUSS_SPEC, 9, 512, 1, 120), (U.MOD_POINT, 64, 256, 2, 20)]):
+        uv, sky = small(mt, nrow=nrow, nchan=nchan, nif=nif, ncomp=ncomp, dnu=1e8 / (nchan * nif), seed=60 + i)
+        d, c = torch.from_numpy(uv.vis.copy()).cuda(), torch.from_numpy(sky.comps).cuda()
+        keep.append((d, c))
+        cases.append((uv, sky))
+        facets.append(Facet(uv, sky, SkyModelParams(op=OP_SUB), d.data_ptr(), nrow, c.data_ptr()))
+    b = DFTBatch(facets)
+    try:
+        host = [torch.from_numpy(uv.vis.copy()).pin_memory() for uv, _ in cases]
+        b.run()
+        b.check()
+        b.run_host([h.data_ptr() for h in host], 1 << 20)
+        b.check()
+        for (uv, sky), (d, _), h in zip(cases, keep, host):
+            got = d.cpu().numpy()
+            assert np.array_equal(got, h.numpy())
+            _, l1 = oracle.model_fp64(uv, sky)
+            want = oracle.apply_fp64(uv, sky, SkyModelParams(op=OP_SUB))
+            err = np.abs(got - want)[:, uv.nrparm:].reshape(uv.vis_view().shape)[..., :2, :2]
+            assert (err / l1[..., None, None]).max() < TOL_REL
+    finally:
+        b.close()

@@ -8,62 +8,6 @@ namespace obit {
 
 namespace {
 
-// kMix: a Gaussian-family model whose untapered rows come first as points
-// (p.k.compsPt, p.k.ncompPt).
-template <int MA, int NJ, int T, int EX, bool kCross, int kMix>
-__global__ void __launch_bounds__(32 * T, 12 / T)
-    dft_tc_kernel(const __grid_constant__ TcParams p) {
-  extern __shared__ __align__(16) float smem[];
-  float* sTab = smem;
-  float2* sScale = reinterpret_cast<float2*>(sTab + T * tc_tab_floats(NJ, T));
-  float2* sL2 = sScale + 2 * T * T;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int g = lane >> 2, t = lane & 3;
-  const long long nItems = (long long)p.k.nvis * p.nteam;
-  for (long long item = blockIdx.x; item < nItems; item += gridDim.x) {
-    const int row = (int)(item / p.nteam);
-    const TcTeamDesc& tm = p.teams[item - (long long)row * p.nteam];
-    float* rec = p.k.vis + (size_t)(p.k.rowBase + row) * p.k.lrec;
-    const float u = rec[p.k.ilocu], v = rec[p.k.ilocv], w = rec[p.k.ilocw];
-    TcSums<MA, NJ> S;
-#pragma unroll
-    for (int i = 0; i < MA * NJ * 4; i++) (&S.tot[0][0][0][0])[i] = 0ull;
-    if constexpr (kMix != 0)
-      tc_pass<MA, NJ, T, kExSpec, (kMix == 2), false>(p, tm, p.k.compsPt, nullptr, p.k.ncompPt, 4, u, v, w, sTab, sScale,
-                                               sL2, S);
-    tc_pass<MA, NJ, T, EX, kCross, false>(p, tm, p.k.comps, p.k.compsLo, p.k.ncomp, p.specField, u, v, w, sTab, sScale, sL2,
-                                   S);
-    // every warp has read u, v, w and applies its own channels
-    const TcSeg& seg = tm.seg[warp];
-#pragma unroll
-    for (int mi = 0; mi < MA; mi++)
-#pragma unroll
-      for (int j = 0; j < NJ; j++)
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-          const int a = 16 * mi + g + 8 * (e >> 1), n = 8 * j + 2 * t + (e & 1);
-          const int ch = seg.ch0 + tm.D * a + n;
-          float sr, si;
-          {
-            float x[2], y[2];
-            up2(S.tot[mi][j][0][e >> 1], x[0], x[1]);
-            up2(S.tot[mi][j][1][e >> 1], y[0], y[1]);
-            sr = x[e & 1];
-            si = y[e & 1];
-          }
-          if (S.merged) {
-            const int i0 = ((mi * NJ + j) * 2) * 4 + e;
-            const float2 lr = sL2[i0 * (32 * T) + threadIdx.x], li = sL2[(i0 + 4) * (32 * T) + threadIdx.x];
-            sr = lr.x + (lr.y + sr);
-            si = li.x + (li.y + si);
-          }
-          if (ch < seg.end) apply_channel(p.k, rec + p.chanOff[ch], sr, si);
-        }
-  }
-}
-
-using TcFn = void (*)(const TcParams);
-
 template <int MA, int NJ, int T>
 TcFn tc_pick_shape(int kind, bool crossPt, int mixed) {
   switch (kind) {
@@ -79,6 +23,7 @@ TcFn tc_pick_shape(int kind, bool crossPt, int mixed) {
 }
 
 TcFn tc_pick(const TcPlan& pl) {
+  if (pl.kind == kPointTSpec || pl.kind == kGaussTSpec) return tc_pick_tab(pl);
   if (pl.MA == 2 && pl.NJ == 2 && pl.T == 2) return tc_pick_shape<2, 2, 2>(pl.kind, pl.crossPt, pl.mixed);
   if (pl.MA == 2 && pl.NJ == 2 && pl.T == 1) return tc_pick_shape<2, 2, 1>(pl.kind, pl.crossPt, pl.mixed);
   if (pl.MA == 1 && pl.NJ == 2 && pl.T == 1) return tc_pick_shape<1, 2, 1>(pl.kind, pl.crossPt, pl.mixed);
@@ -126,7 +71,7 @@ int tc_finalize(TcPlan* plan, const KParams& base, std::string* err) {
   q.chanOff = reinterpret_cast<const int*>(d + bt16);
   q.expo = reinterpret_cast<const float*>(d + bt16 + bc);
   q.lay = tc_expo_layout(plan->MA, plan->NC);
-  q.specField = (plan->kind == kGaussSpec) ? 7 : kSpecIndexField;
+  q.specField = (plan->kind == kGaussSpec || plan->kind == kGaussTSpec) ? 7 : kSpecIndexField;
   return 0;
 }
 

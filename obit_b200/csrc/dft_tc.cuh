@@ -51,6 +51,7 @@ namespace {
 
 // Exponent terms of an instance.
 constexpr int kExNone = 0, kExSpec = 1, kExGauss = 2, kExBoth = 3;
+constexpr int kExTab = 4;  // fluxes tabulated per coarse plane (with kExSpec)
 
 constexpr int kEntry = 80;         // floats per table entry: 16 pairs x 4 and padding (see tc_tab)
 constexpr int kEntW = 0, kEntS = 8, kEntW8 = 16, kEntExp = 17, kEntAnchor = 18;
@@ -224,8 +225,8 @@ __device__ __forceinline__ void tc_pass(const TcParams& p, const TcTeamDesc& tm,
                                         TcSums<MA, NJ>& S, const BeamKParams* bm = nullptr,
                                         const int* perm = nullptr, int ta = 0, int tc = 0) {
   static_assert(!kBeam || T == 1, "a beam's segments lie in one Jones plane each");
-  constexpr bool kSpec = (EX & kExSpec) != 0, kGau = (EX & kExGauss) != 0;
-  constexpr int kTab = tc_tab_floats(NJ, T);
+  constexpr bool kSpec = (EX & kExSpec) != 0, kGau = (EX & kExGauss) != 0, kTab = (EX & kExTab) != 0;
+  constexpr int kTabF = tc_tab_floats(NJ, T);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
   const TcSeg& seg = tm.seg[warp];
@@ -234,12 +235,14 @@ __device__ __forceinline__ void tc_pass(const TcParams& p, const TcTeamDesc& tm,
   // this lane's row and column constants
   float lamR[2 * MA], xiR[2 * MA], xlR[2 * MA], xfR[2 * MA], lamC[NJ], xiC[NJ];
   uint32_t yC[NJ];
+  int fieldR[kTab ? 2 * MA : 1];  // table field of the rows' plane fluxes
 #pragma unroll
   for (int i = 0; i < 2 * MA; i++) {
     lamR[i] = kSpec ? ex[p.lay.lamRow + 8 * i + g] : 0.f;
     xiR[i] = kGau ? ex[p.lay.xiRow + 8 * i + g] : 0.f;
     xlR[i] = (kCross && kSpec) ? ex[p.lay.xl + 8 * i + g] : 0.f;
     xfR[i] = (kCross && kGau) ? ex[p.lay.xf + 8 * i + g] : 0.f;
+    if constexpr (kTab) fieldR[i] = specField + 1 + __float_as_int(ex[p.lay.plane + 8 * i + g]);
   }
 #pragma unroll
   for (int j = 0; j < NJ; j++) {
@@ -250,7 +253,7 @@ __device__ __forceinline__ void tc_pass(const TcParams& p, const TcTeamDesc& tm,
   }
 
   {  // power 0 of both steps: one, for every component
-    float* tb = sTab + warp * kTab + lane * 2;
+    float* tb = sTab + warp * kTabF + lane * 2;
     *reinterpret_cast<float2*>(tb + (kEntW + 4) * kEntry) = *reinterpret_cast<float2*>(tb + (kEntS + 4) * kEntry) =
         ((lane & 1) ^ (lane >> 4)) ? make_float2(0.f, 0.f) : make_float2(1.f, 1.f);
   }
@@ -282,7 +285,7 @@ __device__ __forceinline__ void tc_pass(const TcParams& p, const TcTeamDesc& tm,
       // (the second half of the pairs holds {im, im, re, re}: the 32 lanes' stores
       // fall on 32 banks)
       const int half = lane >> 4;
-      float* tb = sTab + warp * kTab + ((lane >> 3) * 4 + (lane & 3)) * 4 + ((lane >> 2) & 1) + 2 * half;
+      float* tb = sTab + warp * kTabF + ((lane >> 3) * 4 + (lane & 3)) * 4 + ((lane >> 2) & 1) + 2 * half;
       const int im0 = half ? -2 : 2;
       auto put = [&](int e, float re, float im) {
         tb[e * kEntry] = re;
@@ -350,11 +353,17 @@ __device__ __forceinline__ void tc_pass(const TcParams& p, const TcTeamDesc& tm,
       for (int q = 0; q < T; q++) {
         const TcSeg& sg = tm.seg[q];
         float amp = A;
+        if constexpr (kTab) {  // the rows carry the planes' fluxes; the scale is their largest
+          amp = have ? 1.f : 0.f;
+          A = 0.f;
+          const float* sp = comps + (size_t)(have ? c : 0) * p.k.cstride + specField + 1;
+          for (int pl = sg.plane0; pl <= sg.plane1; pl++) A = fmaxf(A, fabsf(__ldg(sp + pl)));
+        }
         if constexpr (kSpec || kGau) {
           float e = 0.f;
           if constexpr (kSpec) e = al * sg.lam0;
           if constexpr (kGau) e = __fmaf_rn(Q, sg.xi0, e);
-          amp = A * expf(e);
+          amp = (kTab ? amp : A) * expf(e);
         }
         float cr[4], ci[4], big = amp;
         if constexpr (kBeam) {
@@ -376,8 +385,15 @@ __device__ __forceinline__ void tc_pass(const TcParams& p, const TcTeamDesc& tm,
         const uint32_t m = __reduce_max_sync(0xffffffffu, __float_as_uint(big) & 0x7fffffffu);
         const int e2 = min(max((int)(m >> 23), 1), 253);
         const float up = __uint_as_float((uint32_t)(254 - e2) << 23);
-        if (lane == 0) sScale[warp * T + q] = make_float2(__uint_as_float((uint32_t)e2 << 23), at);
+        const float inv = __uint_as_float((uint32_t)e2 << 23);
         amp *= up;
+        if constexpr (kTab) {  // the fluxes on H have a scale of their own
+          const uint32_t ms = __reduce_max_sync(0xffffffffu, __float_as_uint(have ? A : 0.f));
+          const int es = min(max((int)(ms >> 23), 1), 253);
+          const float upS = __uint_as_float((uint32_t)(254 - es) << 23);
+          if (lane == 0) sScale[T * T + warp * T + q] = make_float2(upS, __uint_as_float((uint32_t)es << 23));
+        }
+        if (lane == 0) sScale[warp * T + q] = make_float2(inv, at);
         float zr = amp * ar[q], zi = amp * ai[q];
 #pragma unroll
         for (int j = 0; j < NJ; j++) {
@@ -403,7 +419,10 @@ __device__ __forceinline__ void tc_pass(const TcParams& p, const TcTeamDesc& tm,
       for (int i = 0; i < MA * NJ * 8; i++) (&acc[0][0][0][0])[i] = 0.f;
       const float2 sc = sScale[q * T + warp];
       const float at = sc.y;
-      const float* tb = sTab + q * kTab + t * 4;
+      const float2 fl = kTab ? sScale[T * T + q * T + warp] : make_float2(1.f, 1.f);  // the fluxes' scale and its inverse
+      const float up = fl.x;
+      const int cq = base + kTcChunk * q + t;
+      const float* tb = sTab + q * kTabF + t * 4;
       // ---- 4 steps of 8 components.  The fragments of the next step are formed
       // between the products of this one: stage i is a row (pair of fragment
       // registers per component) or a column group, and a group of products
@@ -428,7 +447,7 @@ __device__ __forceinline__ void tc_pass(const TcParams& p, const TcTeamDesc& tm,
         // exponent x on (zr, zi): to first order where the indices of a chunk are
         // close (the planner's bound), else exp(x)
         auto grow = [&](f2x x, f2x& zr, f2x& zi) {
-          if constexpr (EX == kExSpec && !kCross) {
+          if constexpr (!kGau && !kCross) {
             zr = fma2(zr, x, zr);
             zi = fma2(zi, x, zi);
           } else {
@@ -451,6 +470,13 @@ __device__ __forceinline__ void tc_pass(const TcParams& p, const TcTeamDesc& tm,
             if constexpr (kGau) K = fma2(E2, pk2(xfR[r], xfR[r]), K);
           }
           f2x zr = Zr, zi = Zi;
+          if constexpr (kTab) {
+            const float* sp = comps + fieldR[kTab ? r : 0];
+            const int ca = min(cq + 8 * ks, ncomp - 1), cb = min(cq + 8 * ks + 4, ncomp - 1);
+            const f2x S = mul2(pk2(__ldg(sp + (size_t)ca * p.k.cstride), __ldg(sp + (size_t)cb * p.k.cstride)), pk2(up, up));
+            zr = mul2(zr, S);
+            zi = mul2(zi, S);
+          }
           if constexpr (kSpec || kGau) {
             f2x x = 0ull;
             if constexpr (kSpec) x = mul2(E1, pk2(lamR[r], lamR[r]));
@@ -529,12 +555,13 @@ __device__ __forceinline__ void tc_pass(const TcParams& p, const TcTeamDesc& tm,
       for (int mi = 0; mi < MA; mi++)
 #pragma unroll
         for (int j = 0; j < NJ; j++) {
+          const float f0 = kTab ? fl.y : 1.f;  // (two factors: their product may leave the range)
           float f[4] = {sc.x, sc.x, sc.x, sc.x};
           if constexpr (kSpec) {
             const float4 R = __ldg(reinterpret_cast<const float4*>(ex + p.lay.L) + (kBeam ? mi : mi * NJ + j) * 32 + lane);
             const float r[4] = {R.x, R.y, R.z, R.w};
 #pragma unroll
-            for (int e = 0; e < 4; e++) f[e] = sc.x * expf(at * r[e]);
+            for (int e = 0; e < 4; e++) f[e] = sc.x * (kTab ? f0 * expf(at * r[e]) : expf(at * r[e]));
           }
 #pragma unroll
           for (int h = 0; h < 2; h++)
@@ -562,6 +589,60 @@ __device__ __forceinline__ void tc_pass(const TcParams& p, const TcTeamDesc& tm,
         S.merged = true;
       }
     }
+  }
+}
+
+// kMix: a Gaussian-family model whose untapered rows come first as points
+// (p.k.compsPt, p.k.ncompPt).
+template <int MA, int NJ, int T, int EX, bool kCross, int kMix>
+__global__ void __launch_bounds__(32 * T, 12 / T)
+    dft_tc_kernel(const __grid_constant__ TcParams p) {
+  extern __shared__ __align__(16) float smem[];
+  float* sTab = smem;
+  float2* sScale = reinterpret_cast<float2*>(sTab + T * tc_tab_floats(NJ, T));
+  float2* sL2 = sScale + 2 * T * T;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const long long nItems = (long long)p.k.nvis * p.nteam;
+  for (long long item = blockIdx.x; item < nItems; item += gridDim.x) {
+    const int row = (int)(item / p.nteam);
+    const TcTeamDesc& tm = p.teams[item - (long long)row * p.nteam];
+    float* rec = p.k.vis + (size_t)(p.k.rowBase + row) * p.k.lrec;
+    const float u = rec[p.k.ilocu], v = rec[p.k.ilocv], w = rec[p.k.ilocw];
+    TcSums<MA, NJ> S;
+#pragma unroll
+    for (int i = 0; i < MA * NJ * 4; i++) (&S.tot[0][0][0][0])[i] = 0ull;
+    if constexpr (kMix != 0)
+      tc_pass<MA, NJ, T, kExSpec | (EX & kExTab), (kMix == 2), false>(p, tm, p.k.compsPt, nullptr, p.k.ncompPt, 4, u, v, w, sTab, sScale,
+                                               sL2, S);
+    tc_pass<MA, NJ, T, EX, kCross, false>(p, tm, p.k.comps, p.k.compsLo, p.k.ncomp, p.specField, u, v, w, sTab, sScale, sL2,
+                                   S);
+    // every warp has read u, v, w and applies its own channels
+    const TcSeg& seg = tm.seg[warp];
+#pragma unroll
+    for (int mi = 0; mi < MA; mi++)
+#pragma unroll
+      for (int j = 0; j < NJ; j++)
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+          const int a = 16 * mi + g + 8 * (e >> 1), n = 8 * j + 2 * t + (e & 1);
+          const int ch = seg.ch0 + tm.D * a + n;
+          float sr, si;
+          {
+            float x[2], y[2];
+            up2(S.tot[mi][j][0][e >> 1], x[0], x[1]);
+            up2(S.tot[mi][j][1][e >> 1], y[0], y[1]);
+            sr = x[e & 1];
+            si = y[e & 1];
+          }
+          if (S.merged) {
+            const int i0 = ((mi * NJ + j) * 2) * 4 + e;
+            const float2 lr = sL2[i0 * (32 * T) + threadIdx.x], li = sL2[(i0 + 4) * (32 * T) + threadIdx.x];
+            sr = lr.x + (lr.y + sr);
+            si = li.x + (li.y + si);
+          }
+          if (ch < seg.end) apply_channel(p.k, rec + p.chanOff[ch], sr, si);
+        }
   }
 }
 

@@ -22,6 +22,7 @@ struct TcSeg {
   int ch0;             // channel-list index of row 0, column 0; column n is n channels on
   int end;             // first channel-list index past the segment (<= ch0: an empty segment)
   int jplane;          // Jones plane (beam models)
+  int plane0, plane1;  // first and last coarse plane (tabulated spectra)
   int expo;            // float offset of the segment's exponent tables (TcExpo), spectra and tapers
   float lam0, xi0;        // log-frequency term and squared frequency ratio at the reference channel
 };
@@ -37,9 +38,11 @@ struct TcTeamDesc {
 
 // Float offsets inside a segment's exponent tables: the log-frequency term is
 // L(a, n) = lam0 + lamRow(a) + lamCol(n) + R(a, n), the squared frequency ratio
-// xi0 + xiRow(a) + xiCol(n) + xf(a) y(n), and R(a, n) ~ xl(a) y(n).
+// xi0 + xiRow(a) + xiCol(n) + xf(a) y(n), and R(a, n) ~ xl(a) y(n).  (Tabulated
+// spectra: the log frequency is to the row's plane, lam0 = 0, and the rows carry
+// the planes' fluxes.)
 struct TcExpo {
-  int lamRow, xiRow, xl, xf, lamCol, xiCol, y, L, total;
+  int lamRow, xiRow, xl, xf, lamCol, xiCol, y, L, plane, total;
 };
 inline TcExpo tc_expo_layout(int MA, int NJ) {
   TcExpo e{};
@@ -53,6 +56,7 @@ inline TcExpo tc_expo_layout(int MA, int NJ) {
   e.xiCol = take(8 * NJ);
   e.y = take(8 * NJ);
   e.L = take(128 * MA * NJ);  // L(a, n) - lam0, in the order the lanes hold their sums
+  e.plane = take(16 * MA);        // coarse plane of each row (int bits)
   e.total = o;
   return e;
 }
@@ -75,7 +79,7 @@ struct TcPlan {
   bool beam = false;
   int MA = 2, NJ = 2, T = 1;  // 16 MA rows x 8 NJ columns per warp, T warps per team
   int NC = 2;                 // column groups that are channels: NJ, or 1 for a beam (NJ correlations)
-  int kind = kPoint;        // family of the (remaining) table: Point, PointSpec, Gauss, GaussSpec
+  int kind = kPoint;        // family of the (remaining) table
   int mixed = 0;            // a point sub-table precedes the Gaussian rows (as ModelDesc.ncompPt)
   bool crossPt = false;     // point rows with a spectral index need the cross product
   std::vector<TcTeamDesc> teams;
@@ -103,6 +107,10 @@ double tc_recur_cost(const Plan& recur);
 int tc_finalize(TcPlan* plan, const KParams& base, std::string* err);  // plan->beam: the beam kernel
 void tc_free(std::vector<TcPlan>* plan);
 int tc_finalize_all(std::vector<TcPlan>* plan, const KParams& base, std::string* err);
+// Kernels of the tabulated families (dft_tc_tab.cu).
+using TcFn = void (*)(const TcParams);
+TcFn tc_pick_tab(const TcPlan& pl);
+
 struct TcBeamParams {
   TcParams t;
   BeamKParams b;    // antenna types, Jones table, application

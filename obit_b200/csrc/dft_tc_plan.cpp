@@ -4,6 +4,7 @@
 // recurrence kernels.  Plain C++, no CUDA calls.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <functional>
 #include <map>
 
@@ -49,8 +50,9 @@ constexpr Shape kBeamShapes2[] = {{2, 2, 1, 420.0}};
 constexpr Shape kShapes[] = {{2, 2, 2, 792.0}, {2, 2, 1, 416.0}, {1, 2, 1, 261.0}, {1, 1, 1, 192.0}};
 constexpr double kRecurCost = 1.9;
 
-bool spec_kind(int kind) { return kind == kPointSpec || kind == kGaussSpec; }
-bool gauss_kind(int kind) { return kind == kGauss || kind == kGaussSpec; }
+bool tab_kind(int kind) { return kind == kPointTSpec || kind == kGaussTSpec; }
+bool spec_kind(int kind) { return kind == kPointSpec || kind == kGaussSpec || tab_kind(kind); }
+bool gauss_kind(int kind) { return kind == kGauss || kind == kGaussSpec || kind == kGaussTSpec; }
 
 // Half the largest spread of the spectral index within a chunk.
 double chunk_spread(const float* table, int stride, int field, int ncomp) {
@@ -79,15 +81,16 @@ void tc_plan_layout(const LayoutDesc& L, const ModelDesc& M, const float* table,
                     std::vector<TcPlan>* plan, const int* jchan, int ncorr) {
   plan->clear();
   const bool beam = jchan != nullptr;
-  const bool spec = spec_kind(M.kind), gauss = gauss_kind(M.kind);
-  if (!(M.kind == kPoint || M.kind == kGauss || (spec && M.nterm == 1))) return;
+  const bool spec = spec_kind(M.kind), gauss = gauss_kind(M.kind), tab = tab_kind(M.kind);
+  if (!(M.kind == kPoint || M.kind == kGauss || tab || (spec && M.nterm == 1)) || (tab && beam)) return;
   const int npt = M.ncompPt, ntot = npt + M.ncomp;
   if (ntot < kTcMinComps || M.ncomp < 1 || !table) return;
   const int stride = comp_stride(M);
-  const int used = gauss ? (spec ? 8 : 7) : (spec ? 5 : 4);
+  const int planes = tab ? M.nspec : 0;
+  const int used = (gauss ? (spec ? 8 : 7) : (spec ? 5 : 4)) + planes;
   for (int c = 0; c < ntot; c++) {
     const float* r = table + (size_t)c * stride;
-    const int nf = c < npt ? 5 : used;
+    const int nf = c < npt ? 5 + planes : used;
     for (int i = 0; i < nf; i++)
       if (!std::isfinite(r[i])) return;
     // a taper never grows: g1 u^2 + g2 v^2 + g3 u v <= 0 for every u, v
@@ -100,13 +103,15 @@ void tc_plan_layout(const LayoutDesc& L, const ModelDesc& M, const float* table,
   std::vector<double> f;
   std::vector<int> off;
   std::vector<double> ln;
-  std::vector<int> jp;
+  std::vector<int> jp, pl;
   for (int iIF = L.ifb; iIF <= L.ife; iIF++)
     for (int ch = L.chanb; ch <= L.chane; ch++) {
       const int i = ch * L.kincf + iIF * L.kincif;
       f.push_back(L.fscale[i]);
       off.push_back(L.nrparm + iIF * L.incif + ch * L.incf + (beam ? 0 : L.stokb * L.incs));
       jp.push_back(beam ? jchan[i] : 0);
+      pl.push_back(tab ? L.specIndex[i] : 0);
+      if (tab && (pl.back() < 0 || pl.back() >= planes)) return;
       ln.push_back(spec ? L.lnspec[i] : 0.0);
       if (!(L.fscale[i] > 0.0)) return;
     }
@@ -120,11 +125,15 @@ void tc_plan_layout(const LayoutDesc& L, const ModelDesc& M, const float* table,
       // against its mean increment below
       while (e < n && jp[e] == jp[i] && std::fabs(f[e] - (f[i] + (e - i) * df)) <= (1e-13 + 4.5e-16 * (e - i)) * f[i]) e++;
     }
+    // a row of D = 8 or 16 channels lies in one coarse plane: a run ends where
+    // the plane changes inside one
+    for (int k = i + 1; k < e; k++)
+      if (pl[k] != pl[k - 1] && (k - i) % 16 != 0) e = k;
     Run r{f[i], df, i, e - i, spec ? ln[i] - std::log(f[i]) : 0.0, jp[i]};
     if (r.n > 1) r.df = (f[e - 1] - f[i]) / (r.n - 1);
     for (int k = 0; k < r.n; k++) {
       if (std::fabs(f[i + k] - (r.f0 + k * r.df)) > 2e-13 * f[i]) return;
-      if (spec && std::fabs(ln[i + k] - (std::log(f[i + k]) + r.lnShift)) > 1e-9) return;
+      if (spec && !tab && std::fabs(ln[i + k] - (std::log(f[i + k]) + r.lnShift)) > 1e-9) return;
     }
     runs.push_back(r);
     i = e;
@@ -191,29 +200,39 @@ void tc_plan_layout(const LayoutDesc& L, const ModelDesc& M, const float* table,
           p.expo.resize(p.expo.size() + lay.total, 0.0f);
           float* ex = p.expo.data() + g.expo;
           const double nm = 0.5 * (cols - 1);
-          auto Lg = [&](double a, double nn) { return std::log(F(D * a + nn)) + r.lnShift; };
-          auto F2 = [&](double a, double nn) { const double x = F(D * a + nn); return x * x; };
+          // log-frequency term, the row's coarse plane taken from its first channel
           const int last = std::min(r.n - k0, segCap) - 1;          // last valid channel offset
+          auto at = [&](double a) { return r.list0 + k0 + std::min<int>(D * (int)a, last); };
+          auto smooth = [&](double a, double nn) { return std::log(F(D * a + nn)); };
+          auto Lg = [&](double a, double nn) {
+            return smooth(a, nn) + (tab ? ln[at(a)] - std::log(f[at(a)]) : r.lnShift);
+          };
+          auto F2 = [&](double a, double nn) { const double x = F(D * a + nn); return x * x; };
           const double ar = r.df >= 0.0 ? 0.0 : (double)(last / D);  // row of the least taper
           const double am = 0.5 * std::min<double>(rows - 1, (double)(last / D));  // middle valid row
-          const double lam0 = Lg(am, nm), xi0 = F2(ar, nm);
+          const double lam0 = tab ? 0.0 : Lg(am, nm), xi0 = F2(ar, nm);
           g.lam0 = (float)lam0;
           g.xi0 = (float)xi0;
           double yy = 0.0;
           for (int c = 0; c < cols; c++) {
             const double y = (c - nm) * r.df;
             ex[lay.y + c] = (float)y;
-            ex[lay.lamCol + c] = spec ? (float)(Lg(am, c) - lam0) : 0.f;
+            ex[lay.lamCol + c] = spec ? (float)(smooth(am, c) - smooth(am, nm)) : 0.f;
             ex[lay.xiCol + c] = (float)(F2(am, c) - F2(am, nm));
             yy += y * y;
           }
+          g.plane0 = g.plane1 = pl[at(0)];
           for (int a = 0; a < rows; a++) {
+            const int plane = pl[at(a)];
+            g.plane0 = std::min(g.plane0, plane);
+            g.plane1 = std::max(g.plane1, plane);
+            std::memcpy(&ex[lay.plane + a], &plane, sizeof(int));
             ex[lay.lamRow + a] = spec ? (float)(Lg(a, nm) - lam0) : 0.f;
             ex[lay.xiRow + a] = (float)(F2(a, nm) - xi0);
             ex[lay.xf + a] = (float)(2.0 * D * (a - am) * r.df);
             double ry = 0.0, R[64];
             for (int c = 0; c < cols && spec; c++) {
-              R[c] = Lg(a, c) - Lg(a, nm) - Lg(am, c) + lam0;
+              R[c] = smooth(a, c) - smooth(a, nm) - smooth(am, c) + smooth(am, nm);
               ry += R[c] * (c - nm) * r.df;
               // fragment order: lane (row % 8) * 4 + (column % 8) / 2
               const int mi = a >> 4, e = 2 * ((a >> 3) & 1) + (c & 1);

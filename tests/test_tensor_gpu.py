@@ -170,3 +170,19 @@ def test_batch_facets_on_the_tensor_cores():
             assert (err / l1[..., None, None]).max() < TOL_REL
     finally:
         b.close()
+
+
+@pytest.mark.parametrize("mt", [U.MOD_POINT_TSPEC, U.MOD_GAUSS_TSPEC])
+@pytest.mark.parametrize("nchan, nif, nplanes, ncomp", [(256, 1, 4, 300), (512, 2, 16, 1100), (300, 1, 3, 64), (256, 4, 1, 99),
+                                                        (1000, 1, 5, 48)])
+def test_tabulated_spectra(mt, nchan, nif, nplanes, ncomp):
+    """Coarse planes that fall on the grid's rows and ones that cut it, a zero
+    flux and a negative one in a plane."""
+    uv, sky = small(mt, nrow=6, nchan=nchan, nif=nif, ncomp=ncomp, dnu=1.5e8 / (nchan * nif), nplanes=nplanes,
+                    seed=nchan + ncomp, gauss_frac=0.4)
+    first = 5 if mt == U.MOD_POINT_TSPEC else 8
+    sky.comps[3, first] = 0.0
+    sky.comps[5, first:] *= -1.0
+    if mt == U.MOD_POINT_TSPEC and nplanes != 3 and nplanes != 5:
+        assert _plan(uv, sky)["tensorChannels"] > 0
+    assert _error(uv, sky) < TOL_REL

@@ -291,6 +291,15 @@ int plan_layout(const LayoutDesc& L, const ModelDesc& M, const ApplyDesc& A, con
     while (c > 8 && need(c) > budget) c /= 2;
     return c;
   };
+  // A tile is filled to ct components and its (row, component) work done for all
+  // of them, so a tile of the planner's choice is cut to what the table's tiles
+  // hold evenly (13 components at 2 channels, 15,949 records: 11.6 to 9.6 us).
+  auto balanced = [&](int c) {
+    if (T.flavor != kFlavorRecur) return c;
+    const int most = std::max(1, mixed ? std::max(M.ncomp, M.ncompPt) : M.ncomp);
+    const int tiles = (most + c - 1) / c;
+    return std::min(c, std::max(8, ((most + tiles - 1) / tiles + 1) & ~1));
+  };
   // candidate tiles, preferred first: a requested tile shrunk to fit, or the
   // planner's choice (160 components where shared memory holds them as they
   // are: 1 % faster than 128 at configs 2 and 4; else 128 shrunk to fit)
@@ -299,8 +308,8 @@ int plan_layout(const LayoutDesc& L, const ModelDesc& M, const ApplyDesc& A, con
     if (T.ct > 0) {
       c.push_back(fit_from(T.ct));
     } else {
-      if (need(160) <= budget) c.push_back(160);
-      c.push_back(fit_from(128));
+      if (need(160) <= budget) c.push_back(balanced(160));
+      c.push_back(balanced(fit_from(128)));
     }
     return c;
   };

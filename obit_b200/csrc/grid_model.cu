@@ -40,6 +40,7 @@
 #include <vector>
 
 #include "abi_internal.h"
+#include "dft_plan.h"
 #include "grid_host.h"
 #include "obit_dft_grid.h"
 
@@ -349,12 +350,13 @@ __device__ __forceinline__ void conv_setup(float pix, int naxis, int* start, int
   *nterm = iwid - abs(ioff);
 }
 
-// Reference weights from table row itab, taps k0 .. 24, into w[off + i].
-__device__ __forceinline__ float table_weights(const float* __restrict__ tab, int itab, int k0, int nterm,
+// Reference weights from row itab, taps k0 .. 24, of the table in shared memory
+// into w[i].
+__device__ __forceinline__ float table_weights(const float* tab, int itab, int k0, int nterm,
                                                float* w) {
   float s = 0.0f;
   for (int i = 0; i < kGridTaps; i++) {
-    const float v = i < nterm ? __ldg(tab + itab * kGridTaps + k0 + i) : 0.0f;
+    const float v = i < nterm ? tab[itab * kGridTaps + k0 + i] : 0.0f;
     w[i] = v;
     s += v;
   }
@@ -392,30 +394,50 @@ __device__ __forceinline__ float exact_weights(float t, float* w) {
 
 // Rows of a window union summed for G members: this lane's column pair of
 // rows half, half + 2, ... (the other half-warp takes the rest), each row
-// weighted by every member's row weight; members beyond G are zero.
+// weighted by every member's row weight, which lies member by member in the
+// row's 8 floats of wr (one or two 128-bit reads a row); members beyond G are
+// zero.
 template <int G>
 __device__ __forceinline__ void union_rows(const float4* __restrict__ base4, size_t step, int half,
-                                           const float* swb, const int* wo, float4* acc) {
+                                           const float* wr, float4* acc) {
 #pragma unroll
   for (int k = 0; k < kGroup; k++) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
   for (int rr = 0; rr < (kUnion + 1) / 2; rr++) {
     if (2 * rr + half < kUnion) {
       const float4 q = __ldg(base4 + rr * step);
+      float w[kGroup];
+#pragma unroll
+      for (int k = 0; k < G; k += 4)
+        *reinterpret_cast<float4*>(w + k) = *reinterpret_cast<const float4*>(wr + (2 * rr + half) * kGroup + k);
 #pragma unroll
       for (int k = 0; k < G; k++) {
-        const float w = swb[wo[k] + 2 * rr];
-        acc[k].x = fmaf(w, q.x, acc[k].x);
-        acc[k].y = fmaf(w, q.y, acc[k].y);
-        acc[k].z = fmaf(w, q.z, acc[k].z);
-        acc[k].w = fmaf(w, q.w, acc[k].w);
+        acc[k].x = fmaf(w[k], q.x, acc[k].x);
+        acc[k].y = fmaf(w[k], q.y, acc[k].y);
+        acc[k].z = fmaf(w[k], q.z, acc[k].z);
+        acc[k].w = fmaf(w[k], q.w, acc[k].w);
       }
     }
   }
 }
 
+struct ApplySmem {
+  float swr[kApplyWarps][32][kGroup];       // row weights of a group, by union row
+  float sw[kApplyWarps][32][kWX + kWY];     // each lane's weight slots
+  float table[kGridTableRows * kGridTaps];  // the reference's kernel table
+};
+
 __global__ void __launch_bounds__(kApplyWarps * 32, 3) grid_apply_kernel(GridApplyParams p) {
-  __shared__ float sw[kApplyWarps][32][kWX + kWY];
+  extern __shared__ __align__(16) float applySmem[];
+  ApplySmem& sm = *reinterpret_cast<ApplySmem*>(applySmem);
+  auto& sw = sm.sw;
+  auto& swr = sm.swr;
+  if (!p.exact) {
+    // the kernel table: a lane reads 25 consecutive values of a row of its own,
+    // which through L1 cost 32 wavefronts a read
+    for (int i = threadIdx.x; i < kGridTableRows * kGridTaps; i += blockDim.x) sm.table[i] = __ldg(p.table + i);
+    __syncthreads();
+  }
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   float* mywx = sw[wib][lane];
   float* mywy = mywx + kWX;
@@ -470,9 +492,9 @@ __global__ void __launch_bounds__(kApplyWarps * 32, 3) grid_apply_kernel(GridApp
         if (!p.exact) {
           int k0, nt, it;
           conv_setup(px, p.nxp, &sx, &k0, &nt, &it);
-          const float swx = table_weights(p.table, it, k0, nt, wxs);
+          const float swx = table_weights(sm.table, it, k0, nt, wxs);
           conv_setup(py, p.nyp, &sy, &k0, &nt, &it);
-          const float swy = table_weights(p.table, it, k0, nt, wys);
+          const float swy = table_weights(sm.table, it, k0, nt, wys);
           sumwt = swx * swy;
         } else {
           // the requested point itself: 0-relative position px (py) on the plane, a
@@ -523,17 +545,23 @@ __global__ void __launch_bounds__(kApplyWarps * 32, 3) grid_apply_kernel(GridApp
       const int x0e = ux & ~1;
       const float4* base4 = reinterpret_cast<const float4*>(p.plane + (size_t)(uy + half) * p.pitch + x0e) + cp;
       const size_t step = (size_t)p.pitch;  // two rows, in float4
-      // each member's row weight of this lane's first row (slot offsets in the warp's slots)
-      const float* swb = &sw[wib][0][0];
-      int wo[kGroup];
+      // the members' weights of union row `lane`, side by side
+      {
+        const float* swb = &sw[wib][0][0];
+        float wl[kGroup];
 #pragma unroll
-      for (int k = 0; k < kGroup; k++)  // members beyond cnt read lane 0's slots (in range; unused)
-        wo[k] = k < cnt ? mem[k] * (kWX + kWY) + kWX + kSlack - dym[k] + half : kWX;
+        for (int k = 0; k < kGroup; k++)
+          wl[k] = k < cnt ? swb[mem[k] * (kWX + kWY) + kWX + kSlack - dym[k] + min(lane, kUnion - 1)] : 0.f;
+        __syncwarp();  // the previous group's rows have been read
+        *reinterpret_cast<float4*>(&swr[wib][lane][0]) = make_float4(wl[0], wl[1], wl[2], wl[3]);
+        *reinterpret_cast<float4*>(&swr[wib][lane][4]) = make_float4(wl[4], wl[5], wl[6], wl[7]);
+        __syncwarp();
+      }
       float4 acc[kGroup];
       if (cnt <= kGroup / 2)
-        union_rows<kGroup / 2>(base4, step, half, swb, wo, acc);
+        union_rows<kGroup / 2>(base4, step, half, &swr[wib][0][0], acc);
       else
-        union_rows<kGroup>(base4, step, half, swb, wo, acc);
+        union_rows<kGroup>(base4, step, half, &swr[wib][0][0], acc);
       const int cc = x0e + 2 * cp - ux;  // union column of this lane's first value: -1 .. kUnion
       float V[2 * kGroup];                // each member's column-weighted (re, im) of this lane
 #pragma unroll
@@ -750,8 +778,11 @@ int launch_apply(const GridApplyParams& q, cudaStream_t st) {
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   const long long items = (long long)q.nvis * q.nchunk;
   const long long want = (items + kApplyWarps - 1) / kApplyWarps;
-  const int grid = (int)std::min<long long>(want, (long long)nsm * 8);
-  grid_apply_kernel<<<grid, kApplyWarps * 32, 0, st>>>(q);
+  // three resident CTAs per SM, which load the table once
+  const int grid = (int)std::min<long long>(want, (long long)nsm * 3);
+  std::string err;
+  if (int rc = obit::raise_smem_limit((const void*)grid_apply_kernel, sizeof(ApplySmem), &err)) return fail(rc, err);
+  grid_apply_kernel<<<grid, kApplyWarps * 32, sizeof(ApplySmem), st>>>(q);
   CUDA_TRY(cudaGetLastError());
   return OBIT_DFT_OK;
 }

@@ -41,6 +41,7 @@
 
 #include "abi_internal.h"
 #include "dft_plan.h"
+#include "f32x2.cuh"
 #include "grid_host.h"
 #include "obit_dft_grid.h"
 
@@ -400,24 +401,32 @@ __device__ __forceinline__ float exact_weights(float t, float* w) {
 template <int G>
 __device__ __forceinline__ void union_rows(const float4* __restrict__ base4, size_t step, int half,
                                            const float* wr, float4* acc) {
+  using obit::f2x;
+  f2x A[kGroup / 2][4];  // members (2 k, 2 k + 1): the four values of the lane's column pair
 #pragma unroll
-  for (int k = 0; k < kGroup; k++) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int k = 0; k < kGroup / 2; k++) A[k][0] = A[k][1] = A[k][2] = A[k][3] = 0ull;
 #pragma unroll
   for (int rr = 0; rr < (kUnion + 1) / 2; rr++) {
     if (2 * rr + half < kUnion) {
       const float4 q = __ldg(base4 + rr * step);
-      float w[kGroup];
+      const f2x Q[4] = {obit::pk2(q.x, q.x), obit::pk2(q.y, q.y), obit::pk2(q.z, q.z), obit::pk2(q.w, q.w)};
 #pragma unroll
-      for (int k = 0; k < G; k += 4)
-        *reinterpret_cast<float4*>(w + k) = *reinterpret_cast<const float4*>(wr + (2 * rr + half) * kGroup + k);
+      for (int k = 0; k < G; k += 4) {
+        const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(wr + (2 * rr + half) * kGroup + k);
 #pragma unroll
-      for (int k = 0; k < G; k++) {
-        acc[k].x = fmaf(w[k], q.x, acc[k].x);
-        acc[k].y = fmaf(w[k], q.y, acc[k].y);
-        acc[k].z = fmaf(w[k], q.z, acc[k].z);
-        acc[k].w = fmaf(w[k], q.w, acc[k].w);
+        for (int c = 0; c < 4; c++) {
+          A[k / 2][c] = obit::fma2(w.x, Q[c], A[k / 2][c]);
+          A[k / 2 + 1][c] = obit::fma2(w.y, Q[c], A[k / 2 + 1][c]);
+        }
       }
     }
+  }
+#pragma unroll
+  for (int k = 0; k < kGroup / 2; k++) {
+    obit::up2(A[k][0], acc[2 * k].x, acc[2 * k + 1].x);
+    obit::up2(A[k][1], acc[2 * k].y, acc[2 * k + 1].y);
+    obit::up2(A[k][2], acc[2 * k].z, acc[2 * k + 1].z);
+    obit::up2(A[k][3], acc[2 * k].w, acc[2 * k + 1].w);
   }
 }
 

@@ -187,7 +187,7 @@ constexpr int kBlankBits = 0x7fc0beef;
 // come from L2 (1.9 MB at 2 types x 8 planes x 61 x 61 pixels); a warp's load
 // touches 4 units of two rows each.  A thread per (component, type) over all
 // planes, images and taps kept 8,000 threads on 200 dependent loads a plane:
-// 160 us for 4,000 components x 2 types x 8 planes of 61 x 61 pixels, now 41.
+// 160 us for 4,000 components x 2 types x 8 planes of 61 x 61 pixels, now 35.
 constexpr int kJonesThreads = 256;
 constexpr int kMaxCB = 32;
 
@@ -241,36 +241,39 @@ __global__ void __launch_bounds__(kJonesThreads) beam_jones_kernel(const __grid_
       sTap[e] = make_float2(__int_as_float(sFirst[i] + j * p.nx + m), sW[i][0][m] * sW[i][1][j]);
   }
   __syncthreads();
-  const size_t plane = (size_t)p.ny * p.nx;
-  const float* base = p.pixels + (size_t)t * 8 * p.nplane * plane;
-  const int units = nc * p.nplane * 8, l = threadIdx.x & 7;
-  for (int u0 = 0; u0 < units; u0 += kJonesThreads / 8) {
-    const int u = u0 + (threadIdx.x >> 3);
-    const int q = u & 7, ck = u >> 3, i = ck / p.nplane, k = ck - i * p.nplane;
-    const bool have = u < units && sFirst[min(i, CB - 1)] >= 0;
+  // eight lanes per unit: lane group (image q, and a start within the component
+  // and plane pairs), each lane taps l, l + 8, ...
+  const int plane = p.ny * p.nx, l = threadIdx.x & 7, q = (threadIdx.x >> 3) & 7;
+  const float* image = p.pixels + ((size_t)t * 8 + q) * p.nplane * plane;
+  constexpr int kSide = kJonesThreads / 64;  // (component, plane) pairs side by side
+  int i = 0, k = threadIdx.x >> 6;
+  for (int ck0 = 0; ck0 < nc * p.nplane; ck0 += kSide, k += kSide) {
+    while (k >= p.nplane) {
+      k -= p.nplane;
+      i++;
+    }
+    const bool have = i < nc && sFirst[min(i, kMaxCB - 1)] >= 0;
     float sum = 0.f, sumwt = 0.f;
     bool blank = false;
     if (have) {
-      const float* d = base + ((size_t)q * p.nplane + k) * plane;
+      const float* d = image + (size_t)k * plane;
       const float2* tap = sTap + i * ntap;
       for (int e0 = l; e0 < ntap; e0 += 32) {  // four loads in flight per lane
         float val[4], w[4];
 #pragma unroll
-        for (int m = 0; m < 4; m++) {
-          const int e = e0 + 8 * m;
-          const float2 tw = e < ntap ? tap[e] : make_float2(tap[l].x, 0.f);
-          w[m] = tw.y;
+        for (int m = 0; m < 4; m++) {  // (past the last tap: the first again, of no weight)
+          const bool on = e0 + 8 * m < ntap;
+          const float2 tw = tap[on ? e0 + 8 * m : l];
+          w[m] = on ? tw.y : 0.f;
           val[m] = __ldg(d + __float_as_int(tw.x));
         }
 #pragma unroll
         for (int m = 0; m < 4; m++) {
-          if (e0 + 8 * m >= ntap) continue;
-          if (val[m] != p.fblank) {
-            sumwt += w[m];
-            sum += val[m] * w[m];
-          } else {
-            blank = true;
-          }
+          const bool ok = val[m] != p.fblank;
+          blank = blank || !ok;
+          const float wt = ok ? w[m] : 0.f;
+          sumwt += wt;
+          sum += (ok ? val[m] : 0.f) * wt;
         }
       }
     }
@@ -282,7 +285,7 @@ __global__ void __launch_bounds__(kJonesThreads) beam_jones_kernel(const __grid_
       for (int o = 4; o > 0; o >>= 1) sumwt += __shfl_xor_sync(0xffffffffu, sumwt, o);
       wt = sumwt;
     }
-    if (have && l == 0) sV[u] = wt > 0.90f ? sum / wt : __int_as_float(kBlankBits);
+    if (have && l == 0) sV[(i * p.nplane + k) * 8 + q] = wt > 0.90f ? sum / wt : __int_as_float(kBlankBits);
   }
   __syncthreads();
   for (int e = threadIdx.x; e < nc * p.nplane; e += kJonesThreads) {

@@ -767,7 +767,7 @@ def run_beam(args):
                                f"{ntype} antenna types, {njc} Jones planes, Stokes I sky",
                    "rows_per_step": rows, "components": int(sky.ncomp), "channels": 1024,
                    "correlations": ncorr, "l2": "inputs larger than L2", "timing": "CUDA events around all steps",
-                   "beam_form": {0: "blocks, FP32 pipe", 1: "tensor-core (mma.sync TF32, 3-product split)",
+                   "beam_form": {0: "blocks, FP32 pipe", 1: "tensor-core (mma.sync, 3-product split)",
                                  2: "per channel"}[form["form"]], "components_per_tile": form["ct"]},
         "roofline": {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                      "frac": achieved / peak, "traffic": NCU_DRAM_BYTES_PER_RECORD["beam"][0] * rows,
@@ -778,13 +778,12 @@ def run_beam(args):
                      "note": "algorithmic FP32 work of the model (complex rotate + one complex multiply-"
                              "accumulate per correlation); the tensor-core form executes the multiply-"
                              "accumulates as TF32 products (tensor_executed)"},
-        "tensor_executed": ({"tf32_tflops": evals * 96.0 / (statistics.mean(launch_ms) * 1e-3) / 1e12,
-                             "flops_per_eval": 96.0, "what": "3 mma.sync m16n8k8 TF32 products per 64 evaluations "
-                             "(3-product split); ncu puts the pipe at 41 % of its peak on the 4,032-record case"}
+        "tensor_executed": ({"tflops": evals * 96.0 / (statistics.mean(launch_ms) * 1e-3) / 1e12,
+                             "flops_per_eval": 96.0, "what": "three products (f16 in the outer-product form, TF32 "
+                             "in the other) of 16 multiply-accumulates per evaluation"}
                             if form["form"] == 1 else None),
         "comparators": comp, "host": host_info(), "cpu_baseline": None, "e2e": e2e,
-        # the tensor-core form runs its coefficient and amplitude prologues before the kernel
-        "gpu_launches": args.steps * (3 if form["form"] == 1 else 1), "clocks": sampler.summary(),
+        "gpu_launches": args.steps * form["launches"], "clocks": sampler.summary(),
     }
     print(json.dumps(line), flush=True)
     gm.DFTShutdown()
@@ -1134,6 +1133,11 @@ def main():
         pi = gm.plan_info()
         kern = (f"{args.flavor} K={pi['K']} ct={pi['ct']} Bt={pi['Bt']} R={pi['R']} "
                 f"threads={pi['threads']}" + (" spectral-factored" if pi["specFactored"] else ""))
+        tensor = args.flavor == "recur" and pi["tensorChannels"] > 0
+        launches = pi["launches"]
+        if tensor:
+            kern = (f"tensor-core outer-product form, teams of {pi['tensorChannels']} channels "
+                    "(mma.sync f16, operands split hi + lo, 3 products)")
         line = {
             "metric": METRIC,
             "value": value / 1e9, "unit": "Gevals/s", "n_gpus": world, "steps": args.steps,
@@ -1153,12 +1157,17 @@ def main():
                                            + NCU_DRAM_BYTES_PER_RECORD.get(g.name, (0, "no capture"))[1]
                                            + ") x records per launch",
                          "peak_source": "measured here: cuBLAS SGEMM 8192^3, TF32 off (best of 5)",
-                         "flops_per_eval": FLOPS_PER_EVAL},
+                         "flops_per_eval": FLOPS_PER_EVAL,
+                         "note": "the outer-product form's multiply-accumulates run on the tensor cores "
+                                 "(tensor_executed), its phasors on the FP32 pipe" if tensor else None},
+            "tensor_executed": {"f16_tflops": evals * 24.0 / avg_launch_s / 1e12, "flops_per_eval": 24.0,
+                                "what": "three f16 products of 4 multiply-accumulates per evaluation"}
+            if tensor else None,
             "comparators": comp,
             "host": host_info(),
             "cpu_baseline": cpu,
             "e2e": e2e,
-            "gpu_launches": args.steps,
+            "gpu_launches": args.steps * launches,
             "clocks": sampler.summary(),
         }
         print(json.dumps(line), flush=True)

@@ -224,15 +224,18 @@ int obit_dft_set_beam(GPUInfo *gpuInfo, const ObitDFTBeam *beam);
 
 /* The beam kernel the next call will use (building the plan if needed):
  * info[0] = form (0: blocks of at most 8 channels on the FP32 pipe, 1: the
- * tensor-core form -- point families on uniformly spaced channels with the
- * default flavor; OBIT_DFT_RECUR_CHAIN keeps the block form -- 2: one thread
+ * tensor-core forms on uniformly spaced channels with the default flavor, the
+ * outer-product one where runs are long enough and the model has at most one
+ * spectral index; OBIT_DFT_RECUR_CHAIN keeps the block form; 2: one thread
  * per channel, OBIT_DFT_PLAIN), info[1] = components per tile, info[2] =
- * channel runs (form 1) or blocks per record (forms 0 and 2).  Writes
- * min(n, 3) entries; OBIT_DFT_EBADARG when no beam is set.  Form 1 keeps
- * per-plan device tables of the split Jones coefficients and the spectral
- * amplitudes, rewritten at the start of every call (once per obit_dft_calc,
- * before its first chunk), so a Jones table refilled in place between calls
- * is read afresh; calls on one GPUInfo that overlap on the GPU share them. */
+ * channel runs (form 1) or blocks per record (forms 0 and 2), info[3] =
+ * kernel launches of a device-resident call.  Writes min(n, 4) entries;
+ * OBIT_DFT_EBADARG when no beam is set.  The outer-product form reads the
+ * Jones table itself.  The other tensor-core form keeps per-plan device tables
+ * of the split Jones coefficients and the spectral amplitudes, rewritten at the
+ * start of every call (once per obit_dft_calc, before its first chunk), so a
+ * Jones table refilled in place between calls is read afresh; calls on one
+ * GPUInfo that overlap on the GPU share them. */
 int obit_dft_beam_info(GPUInfo *gpuInfo, int *info, int n);
 
 /* Beam images from which the Jones table is interpolated: for every antenna
@@ -312,7 +315,7 @@ int obit_dft_set_tile(GPUInfo *gpuInfo, int blocksPerTile, int threadsPerCTA);
  * (a cudaStream_t; NULL = default stream).  No host copies. */
 int obit_dft_calc_device(GPUInfo *gpuInfo, float *d_vis, int nvis, void *stream);
 
-/* The plan the next call will use (building it if needed): info[0..11] =
+/* The plan the next call will use (building it if needed): info[0..12] =
  * flavor, channels per thread, components per tile, blocks per tile, rows per
  * tile, threads per CTA, channel blocks per row, channel-increment classes;
  * info[8] = 1 when point components with one spectral index take the
@@ -321,9 +324,10 @@ int obit_dft_calc_device(GPUInfo *gpuInfo, float *d_vis, int nvis, void *stream)
  * as spectral-factored points, the rest in the chain form, one launch), and
  * info[10] the number of those point components; info[11] = 0 when these
  * recurrence kernels run, or the channels per team when the tensor-core form
- * takes the call (uniformly spaced runs of 128 channels or more, point and
- * Gaussian families with at most one spectral index, no kernel or tile shape
- * asked for).  Writes min(n, 12) entries. */
+ * takes the call (uniformly spaced runs of some 100 channels or more, point and
+ * Gaussian families with at most one spectral index or fluxes tabulated per
+ * plane, no kernel or tile shape asked for); info[12] = kernel launches of a
+ * device-resident call.  Writes min(n, 13) entries. */
 int obit_dft_plan_info(GPUInfo *gpuInfo, int *info, int n);
 
 /* No counterpart in the reference.  The same model application as

@@ -577,9 +577,14 @@ extern "C" int obit_dft_batch_create(const ObitDFTFacet* in, int nfacet, ObitDFT
     if (md.ncomp < kTcMinComps || f.nvis <= 0) continue;
     Plan p;
     if (plan_layout(f.L, md, f.A, TuneDesc(), &p, &err) || !p.linear) continue;
-    std::vector<float> table((size_t)md.ncomp * comp_stride(md));
-    CUDA_TRY(cudaMemcpy(table.data(), b->d_comps + f.compOff, sizeof(float) * table.size(), cudaMemcpyDeviceToHost));
-    tc_plan_layout(f.L, md, table.data(), tc_recur_cost(p), &f.tc);
+    std::vector<float> table;
+    cudaError_t fetched = cudaSuccess;
+    tc_plan_layout(f.L, md, [&]() -> const float* {
+      table.resize((size_t)md.ncomp * comp_stride(md));
+      fetched = cudaMemcpy(table.data(), b->d_comps + f.compOff, sizeof(float) * table.size(), cudaMemcpyDeviceToHost);
+      return fetched == cudaSuccess ? table.data() : nullptr;
+    }, tc_recur_cost(p), &f.tc);
+    CUDA_TRY(fetched);
     if (int rc = tc_finalize_all(&f.tc, p.kp, &err)) {
       obit_dft_batch_destroy(b.release());
       return fail(rc, err);

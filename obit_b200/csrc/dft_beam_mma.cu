@@ -1,5 +1,6 @@
-// Beam-corrected DFT, tensor-core form (every model family on uniformly
-// spaced channels).
+// Beam-corrected DFT, tensor-core form with a phasor per channel (every model
+// family on uniformly spaced channels; the outer-product form of dft_tc_beam.cu
+// takes longer runs of models with at most one spectral index).
 //
 // The model of record r at channel k for correlation q is
 //   M_q(r, k) = sum_c C_q(pair(r), c, plane) A_c(k) exp(2 pi i P(r, c) f_k):

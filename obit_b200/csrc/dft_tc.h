@@ -1,6 +1,7 @@
 // Tensor-core form of the DFT model (dft_tc.cu): plan types shared by the host
 // planner (dft_tc_plan.cpp, plain C++) and the kernel.
 #pragma once
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -92,14 +93,15 @@ struct TcPlan {
 };
 
 // Host part: whether the tensor-core form takes this layout and model, and its
-// teams and tables.  table: host copy of the table the kernels read (ncompPt
+// teams and tables.  fetch: host copy of the table the kernels read (asked for only
+// when the layout can win; null: recurrence) (ncompPt
 // point rows first when mixed), rows of comp_stride floats.  Leaves *plan
 // empty when the recurrence kernels should run.
 // jchan (beam models): Jones plane per frequency-table index, ncorr modelled
 // correlations; runs never span a change of plane, and recurCost is what the
 // other form costs in the shapes' units.
-void tc_plan_layout(const LayoutDesc& L, const ModelDesc& M, const float* table, double recurCost,
-                    std::vector<TcPlan>* plan, const int* jchan = nullptr, int ncorr = 0);
+void tc_plan_layout(const LayoutDesc& L, const ModelDesc& M, const std::function<const float*()>& fetch,
+                    double recurCost, std::vector<TcPlan>* plan, const int* jchan = nullptr, int ncorr = 0);
 // Cost of the recurrence kernels for a plan of theirs.
 double tc_recur_cost(const Plan& recur);
 

@@ -4,7 +4,9 @@
 // complex products with its Jones coefficients for 128 MA channels and NJ
 // correlations.  The coefficients are formed from the two antennas' Jones
 // matrices once per (record, component, segment), by the lane that holds the
-// component.
+// component.  8,064 records x 1,024 channels x 4,000 points with an index, four
+// correlations, three Jones planes: 17.7 ms against 30.7 of the form with a phasor
+// per channel (dft_beam_mma.cu).
 #include <algorithm>
 
 #include "dft_tc.cuh"

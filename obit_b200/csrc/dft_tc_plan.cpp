@@ -84,27 +84,17 @@ double tc_recur_cost(const Plan& recur) {
   return kRecurCost * recur.kp.nblocks * recur.tune.K;  // its blocks are padded too
 }
 
-void tc_plan_layout(const LayoutDesc& L, const ModelDesc& M, const float* table, double recurCost,
-                    std::vector<TcPlan>* plan, const int* jchan, int ncorr) {
+void tc_plan_layout(const LayoutDesc& L, const ModelDesc& M, const std::function<const float*()>& fetch,
+                    double recurCost, std::vector<TcPlan>* plan, const int* jchan, int ncorr) {
   plan->clear();
   const bool beam = jchan != nullptr;
   const bool spec = spec_kind(M.kind), gauss = gauss_kind(M.kind), tab = tab_kind(M.kind);
   if (!(M.kind == kPoint || M.kind == kGauss || tab || (spec && M.nterm == 1)) || (tab && beam)) return;
   const int npt = M.ncompPt, ntot = npt + M.ncomp;
-  if (ntot < kTcMinComps || M.ncomp < 1 || !table) return;
+  if (ntot < kTcMinComps || M.ncomp < 1) return;
   const int stride = comp_stride(M);
   const int planes = tab ? M.nspec : 0;
   const int used = (gauss ? (spec ? 8 : 7) : (spec ? 5 : 4)) + planes;
-  for (int c = 0; c < ntot; c++) {
-    const float* r = table + (size_t)c * stride;
-    const int nf = c < npt ? 5 + planes : used;
-    for (int i = 0; i < nf; i++)
-      if (!std::isfinite(r[i])) return;
-    // a taper never grows: g1 u^2 + g2 v^2 + g3 u v <= 0 for every u, v
-    if (gauss && c >= npt && !(r[4] <= 0.f && r[5] <= 0.f && 4.0 * r[4] * r[5] >= (double)r[6] * r[6] * (1.0 - 1e-5)))
-      return;
-  }
-
   // ---- uniformly spaced runs of the selected channels -------------------------
   std::vector<Run> runs;
   std::vector<double> f;
@@ -146,7 +136,62 @@ void tc_plan_layout(const LayoutDesc& L, const ModelDesc& M, const float* table,
     i = e;
   }
 
-  // ---- the cheapest shape that holds the bounds ---------------------------------
+  // ---- the cheapest cover of every run by the shapes ------------------------------
+  std::vector<Shape> fit;
+  if (!beam)
+    for (const Shape& s : kShapes) fit.push_back(s);
+  else if (ncorr > 2)
+    for (const Shape& s : kBeamShapes4) fit.push_back(s);
+  else
+    for (const Shape& s : kBeamShapes2) fit.push_back(s);
+  auto capacity = [&](const Shape& s) { return 128 * s.MA * (beam ? 1 : s.NJ) * s.T; };
+  struct Piece {
+    int run, t0;
+  };
+  std::vector<std::vector<Piece>> use;
+  auto cover_runs = [&]() -> double {  // fills use (pieces per shape), returns the cost
+    std::map<int, std::pair<double, int>> cover;  // channels left -> (cost, shape)
+    cover[0] = {0.0, -1};
+    std::function<double(int)> cheapest = [&](int left) -> double {
+      auto it = cover.find(left);
+      if (it != cover.end()) return it->second.first;
+      std::pair<double, int> best{1e300, -1};
+      for (size_t i = 0; i < fit.size(); i++) {
+        const double c = fit[i].cost + cheapest(std::max(0, left - capacity(fit[i])));
+        if (c < best.first) best = {c, (int)i};
+      }
+      cover[left] = best;
+      return best.first;
+    };
+    double cost = 0.0;
+    use.assign(fit.size(), {});
+    for (size_t i = 0; i < runs.size(); i++) {
+      cost += cheapest(runs[i].n);
+      for (int t0 = 0; t0 < runs[i].n;) {
+        const int k = cover[runs[i].n - t0].second;
+        use[k].push_back({(int)i, t0});
+        t0 += capacity(fit[k]);
+      }
+    }
+    return cost;
+  };
+  for (const Run& r : runs)
+    if (r.n > 65536) return;
+  if (!(cover_runs() < recurCost)) return;  // before the table is looked at
+
+  const float* table = fetch();
+  if (!table) return;
+  for (int c = 0; c < ntot; c++) {
+    const float* r = table + (size_t)c * stride;
+    const int nf = c < npt ? 5 + planes : used;
+    for (int i = 0; i < nf; i++)
+      if (!std::isfinite(r[i])) return;
+    // a taper never grows: g1 u^2 + g2 v^2 + g3 u v <= 0 for every u, v
+    if (gauss && c >= npt && !(r[4] <= 0.f && r[5] <= 0.f && 4.0 * r[4] * r[5] >= (double)r[6] * r[6] * (1.0 - 1e-5)))
+      return;
+  }
+
+  // ---- bounds and tables ------------------------------------------------------------
   const double spreadPt = (gauss && npt) || (!gauss && spec)
                               ? chunk_spread(table, stride, kSpecIndexField, gauss ? npt : M.ncomp) : 0.0;
   const float* gt = table + (size_t)npt * stride;
@@ -155,19 +200,7 @@ void tc_plan_layout(const LayoutDesc& L, const ModelDesc& M, const float* table,
   if (!gauss && spec) amax = max_abs(table, stride, kSpecIndexField, M.ncomp);
   if (gauss && npt) amax = max_abs(table, stride, kSpecIndexField, npt);
   if (gauss && spec) amax = std::max(amax, max_abs(gt, stride, 7, M.ncomp));
-  std::vector<Shape> shapes;
-  if (!beam)
-    for (const Shape& s : kShapes) shapes.push_back(s);
-  else if (ncorr > 2)
-    for (const Shape& s : kBeamShapes4) shapes.push_back(s);
-  else
-    for (const Shape& s : kBeamShapes2) shapes.push_back(s);
-  auto capacity = [&](const Shape& s) { return 128 * s.MA * (beam ? 1 : s.NJ) * s.T; };
-
   // Teams of shape s over pieces of runs; false when a bound fails.
-  struct Piece {
-    int run, t0;
-  };
   auto build = [&](const Shape& s, const std::vector<Piece>& pieces, TcPlan* out) -> bool {
     const int NC = beam ? 1 : s.NJ, segCap = 128 * s.MA * NC;
     TcPlan p;
@@ -279,50 +312,22 @@ void tc_plan_layout(const LayoutDesc& L, const ModelDesc& M, const float* table,
     return true;
   };
 
-  // shapes that hold the bounds over whole runs, then the cheapest cover of each
-  // run by them (a run longer than a shape's capacity continues with any shape)
-  std::vector<Shape> fit;
-  for (const Shape& s : shapes) {
-    std::vector<Piece> all;
-    for (size_t i = 0; i < runs.size(); i++)
-      for (int t0 = 0; t0 < runs[i].n; t0 += capacity(s)) all.push_back({(int)i, t0});
-    TcPlan trial;
-    if (build(s, all, &trial)) fit.push_back(s);
-  }
-  if (fit.empty()) return;
-  std::map<int, std::pair<double, int>> cover;  // channels left -> (cost, shape)
-  cover[0] = {0.0, -1};
-  std::function<double(int)> cheapest = [&](int left) -> double {
-    auto it = cover.find(left);
-    if (it != cover.end()) return it->second.first;
-    std::pair<double, int> best{1e300, -1};
-    for (size_t i = 0; i < fit.size(); i++) {
-      const double c = fit[i].cost + cheapest(std::max(0, left - capacity(fit[i])));
-      if (c < best.first) best = {c, (int)i};
+  // a shape that fails a bound is left out and the runs covered by the others
+  while (!fit.empty() && cover_runs() < recurCost) {
+    std::vector<TcPlan> parts;
+    size_t bad = fit.size();
+    for (size_t k = 0; k < fit.size() && bad == fit.size(); k++) {
+      if (use[k].empty()) continue;
+      TcPlan p;
+      if (build(fit[k], use[k], &p)) parts.push_back(std::move(p));
+      else bad = k;
     }
-    cover[left] = best;
-    return best.first;
-  };
-  double cost = 0.0;
-  std::vector<std::vector<Piece>> use(fit.size());
-  for (size_t i = 0; i < runs.size(); i++) {
-    if (runs[i].n > 65536) return;
-    cost += cheapest(runs[i].n);
-    for (int t0 = 0; t0 < runs[i].n;) {
-      const int k = cover[runs[i].n - t0].second;
-      use[k].push_back({(int)i, t0});
-      t0 += capacity(fit[k]);
+    if (bad == fit.size()) {
+      *plan = std::move(parts);
+      return;
     }
+    fit.erase(fit.begin() + bad);
   }
-  if (!(cost < recurCost)) return;
-  std::vector<TcPlan> parts;
-  for (size_t k = 0; k < fit.size(); k++) {
-    if (use[k].empty()) continue;
-    TcPlan p;
-    if (!build(fit[k], use[k], &p)) return;
-    parts.push_back(std::move(p));
-  }
-  *plan = std::move(parts);
 }
 
 }  // namespace obit

@@ -329,14 +329,21 @@ int ensure_plan(GPUInfo* g, State* s) {
   s->plan.kp.compsLo = runLo;
   if (!rc) rc = finalize_plan(&s->plan, nullptr, 0, &err);
   if (rc) return fail(rc, err);
+  // host copy of the run table: prepare_run_table's, or read back when asked for
+  cudaError_t fetched = cudaSuccess;
+  auto fetch = [&]() -> const float* {
+    if (s->runComps == s->d_comps) {
+      table.resize((size_t)md.ncomp * comp_stride(md));
+      fetched = cudaMemcpy(table.data(), s->d_comps, sizeof(float) * table.size(), cudaMemcpyDeviceToHost);
+      if (fetched != cudaSuccess) return nullptr;
+    }
+    return table.data();
+  };
   // the tensor-core form, unless a kernel or tile shape was asked for
   if (T.flavor == kFlavorRecur && T.specFactor && T.K == 0 && T.ct == 0 && T.Bt == 0 && T.threads == 0 &&
       s->plan.linear && !s->beam.on && md.ncompPt + md.ncomp >= kTcMinComps) {
-    if (s->runComps == s->d_comps) {
-      table.resize((size_t)md.ncomp * comp_stride(md));
-      CUDA_TRY(cudaMemcpy(table.data(), s->d_comps, sizeof(float) * table.size(), cudaMemcpyDeviceToHost));
-    }
-    tc_plan_layout(L, md, table.data(), tc_recur_cost(s->plan), &s->tc);
+    tc_plan_layout(L, md, fetch, tc_recur_cost(s->plan), &s->tc);
+    if (fetched != cudaSuccess) return fail(OBIT_DFT_ECUDA, cudaGetErrorString(fetched));
     if ((rc = tc_finalize_all(&s->tc, s->plan.kp, &err))) return fail(rc, err);
   }
   if (s->beam.on) {  // launch parameters and per-(channel, IF) tables of the beam kernel
@@ -374,13 +381,10 @@ int ensure_plan(GPUInfo* g, State* s) {
     bool mma = false;
     if (T.flavor == kFlavorRecur && T.specFactor && T.K == 0 && T.ct == 0 && T.Bt == 0 && T.threads == 0 &&
         s->plan.linear && md.ncompPt + md.ncomp >= kTcMinComps) {
-      if (s->runComps == s->d_comps) {
-        table.resize((size_t)md.ncomp * comp_stride(md));
-        CUDA_TRY(cudaMemcpy(table.data(), s->d_comps, sizeof(float) * table.size(), cudaMemcpyDeviceToHost));
-      }
       const int ncorr = L.nstok >= 4 ? 4 : std::min(2, L.nstok);
       long long nch = (long long)(L.chane - L.chanb + 1) * (L.ife - L.ifb + 1);
-      tc_plan_layout(L, md, table.data(), kBeamMmaCost * (double)nch, &s->tc, b.jchan.data(), ncorr);
+      tc_plan_layout(L, md, fetch, kBeamMmaCost * (double)nch, &s->tc, b.jchan.data(), ncorr);
+      if (fetched != cudaSuccess) return fail(OBIT_DFT_ECUDA, cudaGetErrorString(fetched));
       if (!s->tc.empty()) {
         if ((rc = tc_finalize_all(&s->tc, s->plan.kp, &err))) return fail(rc, err);
         if (s->runComps == s->d_sorted && (rc = upload(order.data(), sizeof(int) * order.size(), (void**)&b.d_perm)))
@@ -786,10 +790,11 @@ int obit_dft_plan_info(GPUInfo* g, int* info, int n) {
   rc = ensure_plan(g, s);
   if (rc) return rc;
   const Plan& pl = s->plan;
-  const int v[12] = {pl.tune.flavor, pl.tune.K, pl.kp.ct, pl.kp.Bt, pl.kp.R, pl.threads,
+  const int v[13] = {pl.tune.flavor, pl.tune.K, pl.kp.ct, pl.kp.Bt, pl.kp.R, pl.threads,
                      pl.kp.nblocks, pl.kp.ndf, pl.specFactored ? 1 : 0, pl.mixed ? 1 : 0,
-                     pl.mixed ? pl.model.ncompPt : 0, s->tc.empty() ? 0 : 128 * s->tc[0].MA * s->tc[0].NJ * s->tc[0].T};
-  for (int i = 0; i < n && i < 12; i++) info[i] = v[i];
+                     pl.mixed ? pl.model.ncompPt : 0, s->tc.empty() ? 0 : 128 * s->tc[0].MA * s->tc[0].NJ * s->tc[0].T,
+                     std::max(1, (int)s->tc.size())};
+  for (int i = 0; i < n && i < 13; i++) info[i] = v[i];
   return OBIT_DFT_OK;
 }
 
@@ -806,9 +811,10 @@ int obit_dft_beam_info(GPUInfo* g, int* info, int n) {
   const bool outer = !s->tc.empty();
   int teams = 0;
   for (const TcPlan& part : s->tc) teams += (int)part.teams.size();
-  const int v[3] = {outer || k.mma ? 1 : (k.flavor == kFlavorPlain ? 2 : 0), outer ? kTcChunk : k.k.ct,
-                    outer ? teams : k.mma ? k.nseg : k.k.nblocks};
-  for (int i = 0; i < n && i < 3; i++) info[i] = v[i];
+  const int v[4] = {outer || k.mma ? 1 : (k.flavor == kFlavorPlain ? 2 : 0), outer ? kTcChunk : k.k.ct,
+                    outer ? teams : k.mma ? k.nseg : k.k.nblocks,
+                    outer ? (int)s->tc.size() : !k.mma ? 1 : k.ampTab ? 3 : 2};
+  for (int i = 0; i < n && i < 4; i++) info[i] = v[i];
   return OBIT_DFT_OK;
 }
 

@@ -193,19 +193,19 @@ class GPUSkyModel:
 
     def plan_info(self) -> dict:
         """The kernel plan the next call uses (built on demand)."""
-        arr = (C.c_int * 12)()
-        _lib.check(self._lib.obit_dft_plan_info(self.gpuinfo, arr, 12))
+        arr = (C.c_int * 13)()
+        _lib.check(self._lib.obit_dft_plan_info(self.gpuinfo, arr, 13))
         keys = ("flavor", "K", "ct", "Bt", "R", "threads", "nblocks", "ndf", "specFactored", "mixed",
-                "ncompPoint", "tensorChannels")
+                "ncompPoint", "tensorChannels", "launches")
         return dict(zip(keys, list(arr)))
 
     def beam_info(self) -> dict:
         """The beam kernel the next call uses: form 0 (blocks on the FP32
         pipe), 1 (tensor-core form) or 2 (one thread per channel), components
-        per tile, channel runs or blocks per record."""
-        arr = (C.c_int * 3)()
-        _lib.check(self._lib.obit_dft_beam_info(self.gpuinfo, arr, 3))
-        return dict(zip(("form", "ct", "units"), list(arr)))
+        per tile, channel runs or blocks per record, kernels per device call."""
+        arr = (C.c_int * 4)()
+        _lib.check(self._lib.obit_dft_beam_info(self.gpuinfo, arr, 4))
+        return dict(zip(("form", "ct", "units", "launches"), list(arr)))
 
     def calc_device(self, d_vis_ptr: int, nvis: int, stream_ptr: int = 0) -> None:
         """Apply the model to nvis records already in device memory (async)."""

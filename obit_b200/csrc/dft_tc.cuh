@@ -21,7 +21,7 @@
 // Programmability, Performance & Precision", 2018).  Phasors are at most 1 and
 // G carries the amplitude scaled by a power of two per chunk of 32 components,
 // so what is dropped is below 2^-23 of the chunk's largest amplitude.  The
-// tensor cores truncate when they add, so the sums of a chunk (24 products)
+// tensor cores truncate when they add, so the sums of a chunk (12 products)
 // are added to FP32 totals by the lanes, and those every kMergeChunks chunks
 // to compensated ones.
 //
@@ -265,6 +265,9 @@ __device__ __forceinline__ void tc_pass(const TcParams& p, const TcTeamDesc& tm,
     *reinterpret_cast<float2*>(tb + (kEntW + 4) * kEntry) = *reinterpret_cast<float2*>(tb + (kEntS + 4) * kEntry) =
         ((lane & 1) ^ (lane >> 4)) ? make_float2(0.f, 0.f) : make_float2(1.f, 1.f);
   }
+  // the lowest squared frequency ratio of the team (a team's last segments may be empty)
+  const float xiMin =
+      (T > 1 && tm.seg[T - 1].ch0 < tm.seg[T - 1].end) ? fminf(tm.seg[0].xi0, tm.seg[T - 1].xi0) : tm.seg[0].xi0;
   for (int base = 0; base < ncomp; base += kTcChunk * T) {
     __syncthreads();  // the previous chunks' readers are done with the tables
     {
@@ -280,7 +283,7 @@ __device__ __forceinline__ void tc_pass(const TcParams& p, const TcTeamDesc& tm,
         // (a taper below e^-200 is zero in FP32 at every channel: the clamp keeps the
         // cross factors of such components finite in f16)
         if constexpr (kGau)
-          Q = fmaxf(c1.x * u * u + c1.y * v * v + c1.z * u * v, -200.0f / fminf(tm.seg[0].xi0, tm.seg[T - 1].xi0));
+          Q = fmaxf(c1.x * u * u + c1.y * v * v + c1.z * u * v, -200.0f / xiMin);
         if constexpr (kSpec) al = (specField == 4) ? c1.x : c1.w;
       }
       ds P;
